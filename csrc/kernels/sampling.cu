@@ -81,6 +81,12 @@ OGB_DEVICE unsigned long long block_sum_u64(unsigned long long v, unsigned long 
   return r;
 }
 
+OGB_DEVICE unsigned long long warp_sum_u64(unsigned long long v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // Radix select over the weights of one row.  Finds the largest threshold T such that
 //   measure({ i : w[i] >= T }) >= target
 // where measure is the element count (BY_MASS = false, used for top-k) or the summed weight
@@ -97,12 +103,6 @@ struct RadixScratch {
   uint32_t hi[kSampleThreads / 32][kBuckets];
   unsigned long long total[kBuckets];
 };
-
-OGB_DEVICE unsigned long long warp_sum_u64(unsigned long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 
 template <bool BY_MASS>
 OGB_DEVICE uint32_t radix_threshold(const uint32_t* __restrict__ w, int vocab, uint32_t floor_w,
@@ -151,13 +151,14 @@ OGB_DEVICE uint32_t radix_threshold(const uint32_t* __restrict__ w, int vocab, u
     }
     __syncthreads();
     // walk buckets from the top; every thread does the same short walk
-    int chosen = 0;
+    int chosen = -1;
     unsigned long long run = above;
     for (int b = kBuckets - 1; b >= 0; --b) {
       const unsigned long long h = sc.total[b];
       if (run + h >= target) { chosen = b; break; }
       run += h;
     }
+    if (chosen < 0) return floor_w;     // the whole row stays below the target (fewer than k tokens have a weight): no threshold
     above = run;
     prefix |= static_cast<uint32_t>(chosen) << shift;
     __syncthreads();
@@ -275,7 +276,8 @@ sample_kernel(const T* __restrict__ logits, int* __restrict__ out, const float* 
 // ------------------------------------------------------------------------------------------
 // Vectorised variant of sample_kernel: identical arithmetic and results, but every pass over the
 // row uses 16-byte loads (8 logits or 4 weights per thread per iteration), so a pass costs ~4x fewer
-// dependent memory round trips.  Requires vocab % 8 == 0, ld % 8 == 0 and 16-byte aligned rows.
+// dependent memory round trips.  Requires vocab % 8 == 0, ld % 8 == 0 and 16-byte aligned rows.  For vocabularies beyond what a
+// cluster holds (sample_cluster_kernel).
 // ------------------------------------------------------------------------------------------
 template <bool BY_MASS>
 OGB_DEVICE uint32_t radix_threshold_vec(const uint32_t* __restrict__ w, int vocab, uint32_t floor_w,
@@ -338,13 +340,14 @@ OGB_DEVICE uint32_t radix_threshold_vec(const uint32_t* __restrict__ w, int voca
       sc.total[threadIdx.x] = t;
     }
     __syncthreads();
-    int chosen = 0;
+    int chosen = -1;
     unsigned long long run = above;
     for (int b = kBuckets - 1; b >= 0; --b) {
       const unsigned long long h = sc.total[b];
       if (run + h >= target) { chosen = b; break; }
       run += h;
     }
+    if (chosen < 0) return floor_w;     // the whole row stays below the target (fewer than k tokens have a weight): no threshold
     above = run;
     prefix |= static_cast<uint32_t>(chosen) << shift;
     __syncthreads();
@@ -493,6 +496,10 @@ sample_kernel_vec(const __nv_bfloat16* __restrict__ logits, int* __restrict__ ou
   if (threadIdx.x == 0) out[rowi] = (sh_pick >= 0) ? sh_pick : best.i;
 }
 
+}  // namespace ogb
+#include "sampling_cluster.cuh"
+namespace ogb {
+
 // One CTA per sequence: rows [seq*(k+1), seq*(k+1)+k] of the target logits.  Row j predicts the
 // token after draft position j-1 (row 0 follows the last committed token).  accept_len = length of
 // the longest prefix with draft[j] == argmax(row j); out_tokens[seq, 0..accept_len] = the accepted
@@ -595,6 +602,8 @@ extern "C" int ogb_sample_bf16(const void* logits, int* out_tokens, const float*
                                int vocab, int ld, void* stream) {
   if (rows <= 0) return 0;
   if (work == nullptr) return -4;
+  if (sample_cluster_applies(logits, vocab, ld))
+    return launch_sample_cluster(logits, out_tokens, temperature, top_k, top_p, min_p, uniform, rows, vocab, ld, static_cast<cudaStream_t>(stream));
   const bool vec_ok = (vocab % 8 == 0) && (ld % 8 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0) &&
                       ((reinterpret_cast<uintptr_t>(work) & 15) == 0);
   if (vec_ok) {
@@ -661,13 +670,9 @@ extern "C" int ogb_sample_bf16_no_alloc(const void* logits, int* out_tokens, con
     if (e != cudaSuccess) return static_cast<int>(e);
     g_no_alloc_work_ptr[dev] = static_cast<uint32_t*>(p);
   }
-  // same choice as ogb_sample_bf16: the vectorised kernel when rows are 16-byte aligned (the array itself is
-  // 256-byte aligned and a row of it starts at a multiple of vocab * 4 bytes); both kernels pick identical tokens
-  const bool vec_ok = (vocab % 8 == 0) && (ld % 8 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0);
-  if (vec_ok) {
-    sample_kernel_vec<<<rows, kSampleThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(logits), out_tokens, temperature, top_k, top_p, min_p, uniform,
-        g_no_alloc_work_ptr[dev], vocab, ld);
+  // same choice as ogb_sample_bf16 (kNoAllocMaxVocab logits always fit the cluster); both kernels pick identical tokens
+  if (sample_cluster_applies(logits, vocab, ld)) {
+    return launch_sample_cluster(logits, out_tokens, temperature, top_k, top_p, min_p, uniform, rows, vocab, ld, static_cast<cudaStream_t>(stream));
   } else {
     sample_kernel<<<rows, kSampleThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(logits), out_tokens, temperature, top_k, top_p, min_p, uniform,
