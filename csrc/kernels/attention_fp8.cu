@@ -12,6 +12,7 @@
 //   scale  K scale multiplies the scores of the page's 16 keys, V scale multiplies their
 //          probabilities before P.V; the running row sum uses the unscaled probabilities
 // Head dimension 128 only.  Same bounded waits and status word as the bf16 kernels.
+#include <cooperative_groups.h>
 #include <cuda_fp8.h>
 
 #include <cstdlib>
@@ -119,14 +120,19 @@ OGB_DEVICE bool fp8_produce(const CUtensorMap* kv_map, const AttnParams& p, uint
   int stage = 0;
   uint32_t phase = 0;
   for (int b = b_begin; b < b_end; ++b) {
+    int64_t page_of_slot[4];             // read ahead of the wait for the slot
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      int pi = min(min(b * 4 + i, n_pages - 1), p.max_pages - 1);
+      pi = skip_gap_page(pi, p.window, p.sink, kv_lo);
+      page_of_slot[i] = table[pi];
+    }
     if (!mbar_wait(&empty_bar[stage], phase ^ 1)) return false;
     uint8_t* s = stages + stage * kRawStage;
     mbar_expect_tx(&full_bar[stage], kRawStage);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      int pi = min(min(b * 4 + i, n_pages - 1), p.max_pages - 1);
-      pi = skip_gap_page(pi, p.window, p.sink, kv_lo);
-      int64_t page = table[pi];
+      int64_t page = page_of_slot[i];
       if (page < 0 || page >= p.num_pages) { atomicOr(p.status, kStatusIndexOutOfRange); page = 0; }
       const int row_k = static_cast<int>(((page * p.hkv + kvh) * 2) * kPageTokens);
       tma_load_2d(s + i * kRawPage, kv_map, &full_bar[stage], 0, row_k);
@@ -701,7 +707,11 @@ __global__ void __maxnreg__(168) paged_decode_e4m3_mma_kernel(const __grid_const
 
 // ------------------------------------------------------------------------------------------
 // prefill (chunked, causal): 64 query rows x one head per CTA; the four consumer warps expand each
-// 64-key block together into one shared bf16 tile
+// 64-key block together into one shared bf16 tile.
+// A tile with at most 32 rows takes 2, 4 or 8 heads of its KV head (64 accumulator rows = heads x 32, 16 or 8 query rows), so a
+// short turn against a long context expands the context once for several heads.  Where that leaves few CTAs, a cluster of
+// num_splits CTAs shares a tile: each walks a part of the keys, then each merges a part of the rows out of all their shared memories
+// (16 rows against 6000 - 12000 tokens, 8 sequences, 28 heads over 4: 1125 -> 290 us; int8, 16 sequences of 300 - 2300: 229 -> 74).
 // ------------------------------------------------------------------------------------------
 constexpr int kPreStages = 2;
 constexpr int kPreTile = kKvBlock * kD * 2;   // 16 KB bf16 K tile (and as much for V)
@@ -719,7 +729,9 @@ __global__ void __launch_bounds__(kAttnThreads) paged_prefill_fp8_kernel(const _
   uint64_t* empty_bar = full_bar + kPreStages;
   float* sc_sh = reinterpret_cast<float*>(empty_bar + kPreStages);   // [4 pages][2]
 
-  const int tile = blockIdx.x;
+  namespace cg = cooperative_groups;
+  const int splits = p.num_splits, split = blockIdx.x % splits;      // the cluster's size and this CTA's place in it
+  const int tile = blockIdx.x / splits;
   if (tile >= p.num_tiles) return;
   const int head = blockIdx.y, kvh = head / p.group;
   const int seq = p.tile_seq[tile], q0 = p.tile_q0[tile];
@@ -729,9 +741,13 @@ __global__ void __launch_bounds__(kAttnThreads) paged_prefill_fp8_kernel(const _
   const int rows = min(64, q_len - q0);
   const int pos0 = ctx - q_len + q0;
   if (rows <= 0 || ctx <= 0) return;
+  const int row_bits = rows > 32 ? 6 : rows > 16 ? 5 : rows > 8 ? 4 : 3;
+  if ((head % p.group) & ((64 >> row_bits) - 1)) return;               // served with an earlier head of the group
+  const int heads_here = min(64 >> row_bits, p.group - head % p.group);
   const int kv_end = min(ctx, pos0 + rows);
   const int kv_lo = (p.window > 0) ? max(0, pos0 - p.window + 1) : 0;   // first key any row of the tile sees in its window
-  const int b_end = (kv_end + kKvBlock - 1) / kKvBlock;
+  const int blocks = (kv_end + kKvBlock - 1) / kKvBlock;
+  const int b_begin = blocks * split / splits, b_end = blocks * (split + 1) / splits;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kPreStages; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 4); }
@@ -740,16 +756,23 @@ __global__ void __launch_bounds__(kAttnThreads) paged_prefill_fp8_kernel(const _
   }
   __syncthreads();
   if (warp == 4) {
-    if (lane == 0 && !fp8_produce(&kv_map, p, stages, full_bar, empty_bar, kPreStages, seq, kvh, ctx, 0, b_end, kv_lo))
+    if (lane == 0 && !fp8_produce(&kv_map, p, stages, full_bar, empty_bar, kPreStages, seq, kvh, ctx, b_begin, b_end, kv_lo))
       atomicOr(p.status, kStatusWaitTimeout);
+    if (splits > 1) {
+      __syncwarp();
+      cg::this_cluster().sync();
+      cg::this_cluster().sync();
+    }
     return;
   }
+  const int row_mask = (1 << row_bits) - 1;
   {
     const __nv_bfloat16* qsrc = p.q + static_cast<size_t>(q_begin + q0) * p.q_stride + head * kD;
     for (int idx = threadIdx.x; idx < 64 * (kD / 8); idx += 128) {
       const int row = idx / (kD / 8), ch = idx % (kD / 8);
       uint4 v = make_uint4(0, 0, 0, 0);
-      if (row < rows) v = *reinterpret_cast<const uint4*>(qsrc + static_cast<size_t>(row) * p.q_stride + ch * 8);
+      if ((row & row_mask) < rows && (row >> row_bits) < heads_here)
+        v = *reinterpret_cast<const uint4*>(qsrc + static_cast<size_t>(row & row_mask) * p.q_stride + (row >> row_bits) * kD + ch * 8);
       *reinterpret_cast<uint4*>(sq + q_tile_off<64>(row, ch * 8)) = v;
     }
   }
@@ -766,22 +789,26 @@ __global__ void __launch_bounds__(kAttnThreads) paged_prefill_fp8_kernel(const _
   for (int j = 0; j < kD / 8; ++j) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
   const int row_a = 16 * warp + (lane >> 2);
-  const int qpos_a = pos0 + row_a, qpos_b = pos0 + row_a + 8;
+  const int qpos_a = pos0 + (row_a & row_mask), qpos_b = pos0 + ((row_a + 8) & row_mask);
   const uint32_t sk = smem_u32(tile_k), sv = smem_u32(tile_v);
 
   int stage = 0;
   uint32_t phase = 0;
   bool ok = true;
-  for (int b = 0; b < b_end; ++b) {
+  // the scales of this warp's page of the coming block, requested one block ahead
+  float sc_next = 0.f;
+  auto request_scale = [&](int b) {
+    if (lane < 2) sc_next = p.kv_scales[(page_of(p, seq, ctx, b * 4 + warp, kv_lo) * p.hkv + kvh) * 2 + lane];
+  };
+  if (b_begin < b_end) request_scale(b_begin);
+  for (int b = b_begin; b < b_end; ++b) {
     if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase))) { ok = false; break; }
     const uint8_t* raw = stages + stage * kRawStage;
     // warp w expands page w of the block (K and V) into the shared bf16 tiles
     expand_page(raw + warp * kRawPage, tile_k + warp * kWorkPage, lane, 32, p.kv_fmt);
     expand_page(raw + (4 + warp) * kRawPage, tile_v + warp * kWorkPage, lane, 32, p.kv_fmt);
-    if (lane < 2) {
-      const int64_t page = page_of(p, seq, ctx, b * 4 + warp, kv_lo);
-      sc_sh[warp * 2 + lane] = p.kv_scales[(page * p.hkv + kvh) * 2 + lane];
-    }
+    if (lane < 2) sc_sh[warp * 2 + lane] = sc_next;
+    if (b + 1 < b_end) request_scale(b + 1);
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty_bar[stage]);   // the raw bytes are no longer needed
     compute_bar_sync();
@@ -853,8 +880,47 @@ __global__ void __launch_bounds__(kAttnThreads) paged_prefill_fp8_kernel(const _
     compute_bar_sync();   // everyone is done with the bf16 tiles before the next block is expanded
     if (++stage == kPreStages) { stage = 0; phase ^= 1; }
   }
-  if (!ok) {
-    if (lane == 0) atomicOr(p.status, kStatusWaitTimeout);
+  if (!ok && lane == 0) atomicOr(p.status, kStatusWaitTimeout);
+  if (splits == 1 && !ok) return;
+  auto out_row = [&](int row) {
+    return p.out + static_cast<size_t>(q_begin + q0 + (row & row_mask)) * p.o_stride + (head + (row >> row_bits)) * kD;
+  };
+  auto stored = [&](int row) { return (row & row_mask) < rows && (row >> row_bits) < heads_here; };
+  if (splits > 1) {
+    // ---- the CTAs of the cluster leave their sums side by side; each merges 64 / splits rows.  The bf16 tiles are idle. ----
+    const cg::cluster_group cluster = cg::this_cluster();
+    float* sm_o = reinterpret_cast<float*>(tile_k);                  // [64][kD]
+    float2* sm_ml = reinterpret_cast<float2*>(stages);               // [64]: maximum, sum (the raw ring is drained)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      float l = l_run[r];
+      l += __shfl_xor_sync(0xffffffffu, l, 1);
+      l += __shfl_xor_sync(0xffffffffu, l, 2);
+      const int row = row_a + 8 * r;
+      if ((lane & 3) == 0) sm_ml[row] = ok ? make_float2(m_run[r], l) : make_float2(-INFINITY, 0.f);
+#pragma unroll
+      for (int j = 0; j < kD / 8; ++j) *reinterpret_cast<float2*>(sm_o + row * kD + 8 * j + 2 * (lane & 3)) = make_float2(o[j][2 * r], o[j][2 * r + 1]);
+    }
+    cluster.sync();
+    const int per = 64 / splits;
+    for (int idx = threadIdx.x; idx < per * (kD / 4); idx += 128) {
+      const int row = split * per + idx / (kD / 4), ch = idx % (kD / 4) * 4;
+      if (!stored(row)) continue;
+      float mx = -INFINITY;
+      for (int c = 0; c < splits; ++c) mx = fmaxf(mx, cluster.map_shared_rank(sm_ml, c)[row].x);
+      float acc[4] = {0.f, 0.f, 0.f, 0.f}, l = 0.f;
+      for (int c = 0; c < splits; ++c) {
+        const float2 ml = cluster.map_shared_rank(sm_ml, c)[row];
+        if (ml.x == -INFINITY) continue;
+        const float w = exp2f(ml.x - mx);
+        const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(sm_o, c) + row * kD + ch);
+        acc[0] += w * v.x; acc[1] += w * v.y; acc[2] += w * v.z; acc[3] += w * v.w;
+        l += w * ml.y;
+      }
+      const float inv = (l > 0.f) ? 1.f / l : 0.f;
+      *reinterpret_cast<uint2*>(out_row(row) + ch) = make_uint2(pack_bf16(acc[0] * inv, acc[1] * inv), pack_bf16(acc[2] * inv, acc[3] * inv));
+    }
+    cluster.sync();                                                  // nobody leaves while its shared memory is being read
     return;
   }
 #pragma unroll
@@ -864,8 +930,8 @@ __global__ void __launch_bounds__(kAttnThreads) paged_prefill_fp8_kernel(const _
     l += __shfl_xor_sync(0xffffffffu, l, 2);
     const float inv = (l > 0.f) ? 1.f / l : 0.f;
     const int row = row_a + 8 * r;
-    if (row < rows) {
-      __nv_bfloat16* dst = p.out + static_cast<size_t>(q_begin + q0 + row) * p.o_stride + head * kD + 2 * (lane & 3);
+    if (stored(row)) {
+      __nv_bfloat16* dst = out_row(row) + 2 * (lane & 3);
 #pragma unroll
       for (int j = 0; j < kD / 8; ++j)
         *reinterpret_cast<uint32_t*>(dst + 8 * j) = pack_bf16(o[j][2 * r] * inv, o[j][2 * r + 1] * inv);
@@ -984,8 +1050,24 @@ static int launch_prefill_q(const void* q, void* out, const void* pool, const fl
     OGB_CUDA_CHECK(cudaFuncSetAttribute(paged_prefill_fp8_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     attr_set = true;
   }
-  paged_prefill_fp8_kernel<<<dim3(num_tiles, hq), kAttnThreads, kPreSmem, static_cast<cudaStream_t>(stream)>>>(map, p);
-  return static_cast<int>(cudaGetLastError());
+  // A tile's CTAs if it has at most 16 rows (longer tiles bring more and have the keys' work to themselves all the same): share
+  // the keys among as many CTAs as two per SM leave room for.  8-byte stores of the merge want an even output stride.
+  const int ctas = num_tiles * hkv * ((p.group + 3) / 4);
+  int splits = 1;
+  while (splits < 8 && 2 * splits * ctas <= 2 * ogb_num_sms() && (o_stride % 4) == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0) splits *= 2;
+  p.num_splits = splits;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(num_tiles * splits, hq);
+  cfg.blockDim = dim3(kAttnThreads);
+  cfg.dynamicSmemBytes = kPreSmem;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = splits;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = splits > 1 ? 1 : 0;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, paged_prefill_fp8_kernel, map, static_cast<AttnParams>(p)));
 }
 
 extern "C" int ogb_paged_decode_fp8(const void* q, void* out, const void* pool, const float* scales, const int* page_table,

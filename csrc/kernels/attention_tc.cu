@@ -151,8 +151,8 @@ OGB_DEVICE float fa_max_chunk(uint32_t s_addr, int hi, int lo) {
 // otherwise [kv_heads][K | V][16][D] with DK = DV = D.
 template <int DK, int DV, int BN, bool CHUNKED>
 __global__ void __launch_bounds__(kFaThreads, 1)
-paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map,
-                        const AttnParams p) {
+paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap q16_map,
+                        const __grid_constant__ CUtensorMap kv_map, const AttnParams p) {
   using Cfg = FaCfg<DK, DV, BN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -178,6 +178,12 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
   const int rows = min(kFaBM, q_len - q0);
   const int pos0 = ctx - q_len + q0;                    // position of the tile's first query row
   if (rows <= 0 || ctx <= 0) return;
+  // A tile with few rows takes several query heads of its KV head: 1 << row_bits tile rows per head.  The later turn of a
+  // conversation -- at most 16 new tokens against a long context -- then reads the context once for 8 heads instead of 8 times
+  // with 16 of 128 rows in use (256 sequences of 614 tokens and 16 rows each, 28 heads over 4: 895 -> 197 us).
+  const int row_bits = CHUNKED || rows > 64 ? 7 : rows > 32 ? 6 : rows > 16 ? 5 : 4;
+  const int heads_here = min(kFaBM >> row_bits, p.group - head % p.group);
+  if ((head % p.group) & ((kFaBM >> row_bits) - 1)) return;        // served with an earlier head of the group
   const int kv_end = min(ctx, pos0 + rows);
   const int kv_lo = (p.window > 0) ? max(0, pos0 - p.window + 1) : 0;
   const int b_begin = kv_lo / BN;
@@ -200,7 +206,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
     }
     *abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&q_map);
+    tma_prefetch_desc(row_bits == 7 ? &q_map : &q16_map);
     tma_prefetch_desc(&kv_map);
   }
   if (warp == 2) {
@@ -220,10 +226,19 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
       FaStamp st{warp == 0 ? dbg : nullptr, 0};
       const bool is_v = (warp == 1);
       if (!is_v) {
-        mbar_expect_tx(&bars->q_full, Cfg::kQBytes);
+        if (row_bits == 7) {
+          mbar_expect_tx(&bars->q_full, Cfg::kQBytes);
 #pragma unroll
-        for (int h = 0; h < Cfg::kHalvesK; ++h)
-          tma_load_2d(sQ + h * Cfg::kHalfStrideQ, &q_map, &bars->q_full, head * (CHUNKED ? p.q_head : DK) + h * 64, q_begin + q0);
+          for (int h = 0; h < Cfg::kHalvesK; ++h)
+            tma_load_2d(sQ + h * Cfg::kHalfStrideQ, &q_map, &bars->q_full, head * (CHUNKED ? p.q_head : DK) + h * 64, q_begin + q0);
+        } else {
+          // rows of a head past its own tokens belong to the next sequence (or are zeros past the buffer): computed, not stored
+          mbar_expect_tx(&bars->q_full, static_cast<uint32_t>(heads_here * Cfg::kHalvesK) * (128u << row_bits));
+          for (int x = 0; x < heads_here; ++x)
+            for (int h = 0; h < Cfg::kHalvesK; ++h)
+              for (int r = 0; r < (1 << row_bits); r += 16)
+                tma_load_2d(sQ + h * Cfg::kHalfStrideQ + (((x << row_bits) + r) << 7), &q16_map, &bars->q_full, (head + x) * DK + h * 64, q_begin + q0 + r);
+        }
       }
       const int n_pages = (ctx + kPageTokens - 1) / kPageTokens;
       const int* table = p.page_table + static_cast<size_t>(seq) * p.max_pages;
@@ -327,11 +342,13 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
     // ------------------------------ softmax groups / correction / epilogue ------------------------------
     const int q = warp & 3;                              // TMEM lane quarter this warp may touch
     const int g = (warp - kFaFirstSoftmaxWarp) >> 2;     // group: 0 takes the even key blocks, 1 the odd ones
-    const int row = q * 32 + lane;                       // query row of this thread
+    const int row = q * 32 + lane;                       // accumulator row of this thread ...
+    const int q_row = row & ((1 << row_bits) - 1), q_head = row >> row_bits;    // ... its query row and its head among the tile's
+    const bool stored = q_row < rows && q_head < heads_here;
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     const uint32_t s_addr = lane_base + Cfg::kColS + g * BN;
     const uint32_t o_addr = lane_base + Cfg::kColO + g * DV;
-    const int qpos = pos0 + row;
+    const int qpos = pos0 + q_row;
     const int hi_abs = min(qpos, ctx - 1);
     const int lo_abs = (p.window > 0) ? (qpos - p.window + 1) : 0;
     float m_run = -INFINITY, l_run = 0.f;                // running maximum in the scaled (log2) domain
@@ -468,13 +485,13 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
         inv *= 1.f / (1.f + __expf(-__bfloat162float(p.gate[static_cast<size_t>(q_begin + q0 + row) * p.ldg + head])));
       const float a = w_mine * inv, b = w_other * inv;
       const float* src = reinterpret_cast<const float*>(xo + (static_cast<size_t>(g ^ 1) * kFaBM + row) * Cfg::kXPitch);
-      __nv_bfloat16* out = p.out + static_cast<size_t>(q_begin + q0 + row) * p.o_stride + head * (CHUNKED ? p.o_head : DV) + g * OC;
+      __nv_bfloat16* out = p.out + static_cast<size_t>(q_begin + q0 + q_row) * p.o_stride + (head + q_head) * (CHUNKED ? p.o_head : DV) + g * OC;
 #pragma unroll
       for (int c = 0; c < OC / 32; ++c) {
         uint32_t o[32];
         tmem_ld_32x32(o_addr + g * OC + 32 * c, o);
         tmem_ld_wait();
-        if (row < rows) {
+        if (stored) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             if (CHUNKED && g * OC + 32 * c + 8 * v >= p.d_v) continue;
@@ -554,9 +571,11 @@ template <int DK, int DV, bool CHUNKED>
 static int launch_prefill_tc(const AttnParams& p, const void* pool, int q_rows, cudaStream_t stream) {
   constexpr int BN = 128;
   using Cfg = FaCfg<DK, DV, BN>;
-  CUtensorMap q_map, kv_map;
-  int rc = cached_tmap(p.q, static_cast<uint64_t>(q_rows), static_cast<uint64_t>(p.hq) * (CHUNKED ? p.q_head : DK), static_cast<uint64_t>(p.q_stride),
-                       kFaBM, &q_map);
+  CUtensorMap q_map, q16_map, kv_map;
+  const uint64_t q_cols = static_cast<uint64_t>(p.hq) * (CHUNKED ? p.q_head : DK);
+  int rc = cached_tmap(p.q, static_cast<uint64_t>(q_rows), q_cols, static_cast<uint64_t>(p.q_stride), kFaBM, &q_map);
+  if (rc != 0) return rc;
+  rc = cached_tmap(p.q, static_cast<uint64_t>(q_rows), q_cols, static_cast<uint64_t>(p.q_stride), 16, &q16_map);
   if (rc != 0) return rc;
   const uint64_t page_rows = static_cast<uint64_t>(p.num_pages) * p.hkv * kPageTokens;
   rc = CHUNKED ? cached_tmap(pool, page_rows * (Cfg::kHalvesK + Cfg::kHalvesV), 64, 64, kPageTokens, &kv_map)
@@ -568,7 +587,7 @@ static int launch_prefill_tc(const AttnParams& p, const void* pool, int q_rows, 
     attr_set = true;
   }
   dim3 grid(p.num_tiles, p.hq);
-  paged_prefill_tc_kernel<DK, DV, BN, CHUNKED><<<grid, kFaThreads, Cfg::kSmemBytes, stream>>>(q_map, kv_map, p);
+  paged_prefill_tc_kernel<DK, DV, BN, CHUNKED><<<grid, kFaThreads, Cfg::kSmemBytes, stream>>>(q_map, q16_map, kv_map, p);
   return static_cast<int>(cudaGetLastError());
 }
 
