@@ -20,10 +20,13 @@
 // drains and frees its TMEM, and the kernel returns.
 #include <stdlib.h>
 
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 
 #include "common.cuh"
+#include "gemm_common.cuh"
+#include "gemm_rows.cuh"
 #include "ogb_kernels.h"
 #include "tp_comm.cuh"
 
@@ -41,37 +44,8 @@ extern "C" int ogb_num_sms() {
 namespace ogb {
 
 constexpr int kBM = 128;
-constexpr int kBK = 64;  // 64 bf16 = one 128-byte swizzle row
 constexpr int kGemmThreads = 192;
 constexpr int kGemmThreadsScatter = 224;  // + one warp that publishes finished tiles to peer GPUs
-
-enum GemmEpilogue : int { kEpiNone = 0, kEpiResidual = 1, kEpiSwiGLU = 2, kEpiScatter = 3 };
-
-// Activations ahead of a bf16 rounding: relative errors of a few 1e-7, absolute ones of 1e-7 next to zero.
-// 0.5 z (1 + tanh(a)) = z / (1 + exp(-2 a))
-OGB_DEVICE float gelu_tanh_fast(float z) {
-  const float a = 0.7978845608028654f * fmaf(0.044715f * z * z, z, z);
-  return z / (1.f + __expf(fminf(-2.f * a, 80.f)));
-}
-// the gated epilogue's value for a gate and an up column
-OGB_DEVICE float gated_act(const ActArgs& act, float g, float u) {
-  if (act.kind == kActGeluTanh) return gelu_tanh_fast(g) * u;
-  if (act.kind == kActClampGlu) {
-    g = fminf(g, act.a);
-    u = fminf(fmaxf(u, -act.a), act.a);
-    return g / (1.f + __expf(fminf(-kClampGluSlope * g, 80.f))) * (u + 1.f);
-  }
-  return g / (1.f + __expf(-g)) * u;
-}
-// the plain epilogue's value for a result
-OGB_DEVICE float plain_act(const ActArgs& act, float v) {
-  if (act.kind == kActRelu2) {
-    v = fmaxf(v, 0.f);
-    return v * v;
-  }
-  if (act.kind == kActXielu) return fmaf(0.5f, v, v > 0.f ? act.a * v * v : act.b * (__expf(v) - 1.f - v));
-  return v;
-}
 
 constexpr int kStagingPitch = 272;                       // bytes per staged row: 128 bf16 + 16 bytes of padding
 constexpr int kStagingWarpBytes = 32 * kStagingPitch;    // one epilogue warp: 32 rows
@@ -84,63 +58,6 @@ struct GemmCfg {
   static constexpr int kStages = (BN >= 256) ? 4 : (BN >= 192 ? 4 : (BN >= 128 ? 6 : 8));
   static constexpr int kTmemCols = (2 * BN <= 32) ? 32 : (2 * BN <= 64 ? 64 : (2 * BN <= 128 ? 128 : (2 * BN <= 256 ? 256 : 512)));  // power of two
   static constexpr int kSmemBytes = kStages * kStage + 256 /*barriers*/ + 4 * kStagingWarpBytes /*epilogue staging*/;
-};
-
-// ----------------------------------------------------------------------------------------
-// Work decomposition.  Data-parallel: output tiles are dealt round-robin to the persistent CTAs and a CTA runs the
-// whole K loop of each of its tiles.  Stream-K: the (tile, k-block) iterations of all tiles are laid end to end and cut
-// into one contiguous, equally long range per CTA, so every SM does the same amount of tensor-core work even when
-// the tile count is not a multiple of the SM count.  A range may begin or end in the middle of a tile: the CTA whose
-// range holds a tile's last k-block finishes the tile; CTAs that hold an earlier part of it leave their fp32
-// accumulator in a workspace slot (one slot per CTA: a range ends inside at most one tile) and raise a flag; the
-// finisher, which always has the higher block index, waits for those flags (bounded) and adds the partials before
-// its epilogue.  Waiting only on lower-numbered CTAs keeps the scheme free of deadlock whatever the residency, and
-// walking every range backwards (GemmWork::next) makes partials the first thing a CTA produces and fix-ups the last.
-// ----------------------------------------------------------------------------------------
-struct GemmSeg {
-  int tile, kb0, kb1;
-};
-
-struct GemmWork {
-  int k_blocks, num_tiles, stride, tile;   // data-parallel cursor
-  long long it, it_end;                    // stream-K cursor over iterations
-  bool sk;
-  OGB_DEVICE static long long range_begin(long long total, int ctas, int b) {
-    const long long base = total / ctas, rem = total % ctas;
-    return b * base + (b < rem ? b : rem);
-  }
-  // the CTA whose range holds iteration i
-  OGB_DEVICE static int owner(long long total, int ctas, long long i) {
-    const long long base = total / ctas, rem = total % ctas;
-    const long long cut = (base + 1) * rem;
-    return i < cut ? static_cast<int>(i / (base + 1)) : static_cast<int>(rem + (i - cut) / base);
-  }
-  OGB_DEVICE GemmWork(bool stream_k, int tiles, int kblocks) : k_blocks(kblocks), num_tiles(tiles), sk(stream_k) {
-    stride = gridDim.x;
-    tile = blockIdx.x;
-    const long long total = static_cast<long long>(tiles) * kblocks;
-    it = stream_k ? range_begin(total, gridDim.x, blockIdx.x) : 0;
-    it_end = stream_k ? range_begin(total, gridDim.x, blockIdx.x + 1) : 0;
-  }
-  OGB_DEVICE bool next(GemmSeg& s) {
-    if (!sk) {
-      if (tile >= num_tiles) return false;
-      s.tile = tile; s.kb0 = 0; s.kb1 = k_blocks;
-      tile += stride;
-      return true;
-    }
-    // The range is walked from its end to its beginning.  The segment at the end of the range is the head of a tile
-    // that a higher-numbered CTA finishes: it is produced first, so the finisher -- for which that tile's tail is the
-    // *last* segment -- finds the partial waiting instead of stalling on a neighbour that has its whole range to go.
-    if (it_end <= it) return false;
-    s.tile = static_cast<int>((it_end - 1) / k_blocks);
-    const long long tile_start = static_cast<long long>(s.tile) * k_blocks;
-    const long long seg_begin = tile_start > it ? tile_start : it;
-    s.kb0 = static_cast<int>(seg_begin - tile_start);
-    s.kb1 = static_cast<int>(it_end - tile_start);
-    it_end = seg_begin;
-    return true;
-  }
 };
 
 // A batch of products that share shapes: problem z reads A from column z * a_step and W from row z * N, and writes its
@@ -851,9 +768,106 @@ static int launch_gemm(const void* A, const void* W, void* C, const void* bias, 
       static_cast<unsigned long long>(a_wait_ns), sk_ws, sk_flags, sk_seq, batch, act));
 }
 
+// ----------------------------------------------------------------------------------------
+// products with few rows (gemm_rows.cuh)
+// ----------------------------------------------------------------------------------------
+// Workspace of the products that one thread launches for a model step: the model's own buffer (its steps follow one another, so its
+// products can share it, replayed graphs included), zeroed when it was made.  Without one -- a call outside a step -- the buffer
+// belongs to the stream, and a capture that finds none takes the tile kernel.
+struct LaunchScope {
+  void* ws = nullptr;
+  size_t bytes = 0;
+};
+static thread_local LaunchScope g_scope;
+
+size_t rows_counter_bytes(int ctas) { return (static_cast<size_t>(ctas) * 4 * sizeof(unsigned int) + 1023) / 1024 * 1024; }
+size_t rows_slot_bytes(int tw, int mn) { return static_cast<size_t>(tw) * 128 * ((mn + 31) / 32 * 32) * sizeof(float); }
+
+void* rows_workspace(cudaStream_t stream, int ctas, int tw, int mn) {
+  const size_t need = rows_counter_bytes(ogb_num_sms()) + 2 * static_cast<size_t>(ctas) * rows_slot_bytes(tw, mn);
+  const size_t most = rows_counter_bytes(ogb_num_sms()) + 2 * static_cast<size_t>(ogb_num_sms()) * rows_slot_bytes(2, kRowsRangesM);
+  if (g_scope.ws != nullptr && g_scope.bytes >= need) return g_scope.ws;
+  static std::mutex mu;
+  static std::unordered_map<uint64_t, void*> table;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  const uint64_t key = (static_cast<uint64_t>(dev) << 56) ^ reinterpret_cast<uint64_t>(stream);
+  std::lock_guard<std::mutex> lock(mu);
+  auto hit = table.find(key);
+  if (hit != table.end()) return hit->second;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return nullptr;
+  void* ws = nullptr;
+  if (cudaMalloc(&ws, most) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  if (cudaMemset(ws, 0, rows_counter_bytes(ogb_num_sms())) != cudaSuccess) { cudaFree(ws); return nullptr; }
+  table.emplace(key, ws);
+  return ws;
+}
+
+template <int TW, int EPI>
+static int launch_rows_one(const void* A, const void* W, int K, int lda, int ldw, RowsGemmParams p, const ActArgs& act, cudaStream_t stream) {
+  auto kernel = gemm_rows_kernel<TW, EPI>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    OGB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmemMax));
+    attr_set = true;
+  }
+  const int sms = ogb_num_sms();
+  const int stage_bytes = TW * 128 * kBK * 2 + p.mn * kBK * 2;
+  p.n_tiles = (p.N + TW * 128 - 1) / (TW * 128);
+  int grid, smem;
+  if (p.n_tiles > sms) {
+    p.splits = 0;
+    grid = sms;
+    p.stages = std::min(kRowsMaxStages, (kRowsSmemMax - kRowsBarBytes - TW * kRowsStage) / stage_bytes);
+    smem = p.stages * stage_bytes + kRowsBarBytes + TW * kRowsStage;
+    void* ws = rows_workspace(stream, grid, TW, p.mn);
+    if (ws == nullptr) return kRowsDeclined;
+    p.counters = static_cast<unsigned int*>(ws);
+    p.ws = reinterpret_cast<float*>(static_cast<char*>(ws) + rows_counter_bytes(sms));
+  } else {
+    // two CTAs per SM where a ring of four stages fits half its shared memory: more parts to choose from
+    const int half = (kRowsSmemMax / 2 - 1024 - kRowsBarBytes) / stage_bytes;
+    p.stages = std::min(kRowsMaxStages, half >= 4 ? half : (kRowsSmemMax - kRowsBarBytes) / stage_bytes);
+    smem = p.stages * stage_bytes + kRowsBarBytes;
+    p.splits = rows_pick_splits(kernel, kRowsThreads, smem, p.n_tiles, p.k_blocks);
+    grid = p.n_tiles * p.splits;
+  }
+  CUtensorMap mw, ma;
+  int rc = make_tmap_bf16_2d(&mw, W, p.N, K, ldw, 128, kBK);
+  if (rc != 0) return rc;
+  rc = make_tmap_bf16_2d(&ma, A, p.M, K, lda, p.mn, kBK);
+  if (rc != 0) return rc;
+  return rows_launch(kernel, grid, kRowsThreads, smem, p.splits, stream, mw, ma, p, act);
+}
+
+// Returns a code, or kRowsDeclined.
+static int launch_rows(const void* A, const void* W, void* C, const void* bias, const void* residual, void* C_f32, int M, int N, int K, int lda, int ldw,
+                       int ldc, int ldr, int epilogue, const ActArgs& act, int* status, cudaStream_t stream) {
+  RowsGemmParams p{};
+  p.mn = (M + 15) / 16 * 16;
+  p.k_blocks = (K + kBK - 1) / kBK;
+  p.C = static_cast<__nv_bfloat16*>(C); p.C_f32 = static_cast<float*>(C_f32);
+  p.bias = static_cast<const __nv_bfloat16*>(bias != nullptr ? bias : W); p.has_bias = bias != nullptr;
+  p.residual = static_cast<const __nv_bfloat16*>(residual);
+  p.M = M; p.N = N; p.ldc = ldc; p.ldr = ldr; p.status = status;
+  if (epilogue == kEpiSwiGLU) return launch_rows_one<2, kEpiSwiGLU>(A, W, K, lda, ldw, p, act, stream);
+  if (epilogue == kEpiResidual) return launch_rows_one<1, kEpiResidual>(A, W, K, lda, ldw, p, act, stream);
+  return launch_rows_one<1, kEpiNone>(A, W, K, lda, ldw, p, act, stream);
+}
+
 }  // namespace ogb
 
 using namespace ogb;
+
+// The buffer that products with few rows use when this thread launches them from now on (null: none).  It starts zeroed, holds
+// ogb_rows_workspace_bytes(rows) and serves one stream at a time.
+extern "C" void ogb_launch_scope(void* ws, int64_t bytes) { g_scope = LaunchScope{ws, static_cast<size_t>(ws != nullptr ? bytes : 0)}; }
+extern "C" int64_t ogb_rows_workspace_bytes(int rows) {
+  const int mn = std::min(kRowsRangesM, (std::max(rows, 1) + 15) / 16 * 16);
+  const int sms = ogb_num_sms();
+  return static_cast<int64_t>(rows_counter_bytes(sms) + 2 * static_cast<size_t>(sms) * rows_slot_bytes(2, mn));
+}
 
 #define OGB_GEMM_ARGS A, W, C, bias, residual, C_f32, M, N, K, lda, ldw, ldc, ldr, status, stream, nullptr, nullptr, nullptr, 1, 0, a_ready, a_done, a_wait_ns, batch, act
 #define OGB_GEMM_DISPATCH_BN(EPI)                              \
@@ -898,6 +912,17 @@ static int gemm_bf16_dispatch(const void* A, const void* W, void* C, const void*
   if (epilogue == kEpiResidual && (residual == nullptr || (ldr % 8) != 0)) return -5;
   if (epilogue == kEpiSwiGLU && (bn < 64 || (N % bn) != 0 || C_f32 != nullptr)) return -6;
   if (batch.count < 1 || (batch.a_step % 8) != 0 || (batch.c_step % 8) != 0 || (batch.count > 1 && (a_ready != nullptr || epilogue != kEpiNone))) return -9;
+  // Few rows: gemm_rows.cuh.  Where the line lies, in us on B200 with weights from HBM, tile kernel -> this one (floor):
+  //   tiles of 128 columns for at most one wave, clusters over K: better at all sizes it takes.  N x K = 4608 x 3584 (5): 26.7 -> 11.2 at 1
+  //     row, 21.5 -> 18.5 at 256; 3584 x 18944 (21): 85.9 -> 29.8, 110 -> 47.1; 128 x 2048: 12.4 -> 5.9, 12.7 -> 10.8
+  //   more tiles, ranges: 152064 x 3584 (169): 225 -> 170 at 1 row, 185 -> 177 at 40, 188 -> 184 at 77, 193 -> 200 at 128; 151936 x 896 (42):
+  //     65 -> 53, 66 -> 63, 54 -> 71, 58 -> 84: the epilogue of a tile is as long as its few k-blocks
+  //   gated 37888 x 3584 (42): 57 -> 49 at 16, 49.2 -> 50.0 at 40, 49.6 -> 53.2 at 77: one tile per SM, whose epilogue nothing hides
+  const int rows_max = epilogue == kEpiSwiGLU ? kRowsGatedM : (N + 127) / 128 > ogb_num_sms() ? kRowsRangesM : kRowsMaxM;
+  if (M <= rows_max && a_ready == nullptr && batch.count == 1 && batch.page_d == 0 && (epilogue == kEpiSwiGLU ? bn == 256 : bn == 0)) {
+    const int rc = launch_rows(A, W, C, bias, residual, C_f32, M, N, K, lda, ldw, ldc, ldr, epilogue, act, status, stream);
+    if (rc != kRowsDeclined) return rc;
+  }
   if (bn == 0) {
     // Tiles are handed out round-robin to one persistent CTA per SM, so the kernel takes
     // ceil(tiles / SMs) "waves" of one tile time each.  Pick the tile width with the lowest

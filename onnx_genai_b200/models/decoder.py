@@ -336,6 +336,8 @@ class DecoderModel:
             self.partial = z(max_tokens, hid)
             self.gate_up = z(max_tokens, 2 * inter_q)
             self.act_q = z(max_tokens, inter_q)
+        # fp32 partials of the products with few rows: one buffer, as the products of a step follow one another
+        self.gemm_ws = ops.rows_workspace(max(max_tokens, max_seqs), dev) if dev.type == "cuda" else None
         self.h_last = z(max_seqs, hid)
         self.x_last = z(max_seqs, hid)
         self.logits = z(max_seqs, cfg.vocab)
@@ -509,6 +511,12 @@ class DecoderModel:
 
     def forward(self, si: StepInputs, kv: KVCache) -> torch.Tensor:
         """Runs one step; returns logits [num_logit_rows, vocab] (a view of a static buffer)."""
+        if self.gemm_ws is None:
+            return self._forward(si, kv)
+        with ops.launch_scope(self.gemm_ws):
+            return self._forward(si, kv)
+
+    def _forward(self, si: StepInputs, kv: KVCache) -> torch.Tensor:
         cfg, w = self.cfg, self.w
         t, nd = si.num_tokens, si.num_decode
         tapping = bool(getattr(self, "tap_layers", None))

@@ -9,6 +9,7 @@ prove which path ran, like the reference's dispatch hit counters (dispatch_manif
 from __future__ import annotations
 
 import collections
+import contextlib
 import math
 import os
 
@@ -244,6 +245,24 @@ def gemm(a, w, bias=None, residual=None, epilogue="none", out=None, out_f32=Fals
     _native.check(rc, "ogb_gemm_bf16")
     launch_counts["gemm_bf16_tcgen05"] += 1
     return out
+
+
+def rows_workspace(rows: int, device) -> torch.Tensor:
+    """The zeroed buffer that products of up to ``rows`` rows keep partial sums in; see :func:`launch_scope`."""
+    with torch.cuda.device(device):
+        n = _native.load().ogb_rows_workspace_bytes(int(rows))
+    return torch.zeros(n, dtype=torch.uint8, device=device)
+
+
+@contextlib.contextmanager
+def launch_scope(workspace: torch.Tensor):
+    """The products that this thread launches inside use ``workspace`` (a model's own: one stream at a time)."""
+    lib = _native.load()
+    lib.ogb_launch_scope(workspace.data_ptr(), workspace.numel())
+    try:
+        yield
+    finally:
+        lib.ogb_launch_scope(0, 0)
 
 
 pack_gate_up = reference.pack_gate_up
