@@ -67,6 +67,7 @@ struct GemmCfg {
 // [16][page_d] and are written there.
 struct GemmBatch {
   int count = 1, a_step = 0, c_step = 0, page_d = 0;
+  int raster = 0;      // tiles in groups of kRasterM tiles of A (raster_tile)
 };
 
 // fp32 partial accumulators of stream-K: slot = CTA, layout [BN / 32 column chunks][128 rows][32 floats], so a warp's
@@ -119,6 +120,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   const int batch_tiles = m_tiles * n_tiles;
   const int num_tiles = batch_tiles * batch.count;
   const int k_blocks = (K + kBK - 1) / kBK;
+  const bool raster = batch.raster != 0;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < Cfg::kStages; ++i) {
@@ -156,8 +158,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       while (ok && work.next(seg)) {
         const int z = seg.tile / batch_tiles;
         const int tile = seg.tile - z * batch_tiles;
-        const int mt = tile % m_tiles;
-        const int n0 = (tile / m_tiles) * BN;
+        int mt, nt;
+        raster_tile(tile, m_tiles, n_tiles, raster, mt, nt);
+        const int n0 = nt * BN;
         const int m0 = group_tab != nullptr ? group_tab[4 * mt + 1] : mt * kBM;
         const int b_row = group_tab != nullptr ? group_tab[4 * mt] * N + n0 : z * N + n0;   // expert e's weights start at row e*N
         const int a_col = z * batch.a_step;
@@ -232,17 +235,17 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     int it = 0;
     GemmWork work(stream_k, num_tiles, k_blocks);
     GemmSeg seg;
-    const long long sk_total = static_cast<long long>(num_tiles) * k_blocks;
+    const long long sk_total = work.sk_total;
     for (; ok && work.next(seg); ++it) {
       const int z = seg.tile / batch_tiles;
       const int tile = seg.tile - z * batch_tiles;
       const size_t c_off = static_cast<size_t>(z) * batch.c_step;
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
-      const int mt = tile % m_tiles;
+      int mt, n_tile;
+      raster_tile(tile, m_tiles, n_tiles, raster, mt, n_tile);
       const int m0 = group_tab != nullptr ? group_tab[4 * mt + 1] : mt * kBM;
       const int m_end = group_tab != nullptr ? group_tab[4 * mt + 2] : M;   // rows past m_end belong to the next expert
-      const int n_tile = tile / m_tiles;
       const int n0 = n_tile * BN;
       // every lane polls (each needs the acquire); the vote keeps the warp converged for tcgen05.ld
       if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full[acc], acc_phase))) { ok = false; break; }
@@ -497,8 +500,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
             if (*abort_flag != 0 || (((++spins) & 0x3ff) == 0 && global_timer_ns() - t0 > kWaitLimitNs)) { ok = false; break; }
           }
           if (!ok) break;
-          const int m0 = (tile % m_tiles) * kBM;
-          const int n0 = (tile / m_tiles) * BN;
+          int mt, nt;
+          raster_tile(tile, m_tiles, n_tiles, raster, mt, nt);
+          const int m0 = mt * kBM;
+          const int n0 = nt * BN;
           const int row0 = m0 + q * 32;
           if (row0 < M) {
             const int owner = row0 / sc->chunk;
@@ -702,20 +707,32 @@ constexpr float kSkFixScatter = 13.0f;
 // A finisher adds the partials of a tile one after the other, so the fix-up grows with the CTAs that share a tile once they are many
 // (8 tiles on 148 SMs, 19 each, took 123 us where whole tiles take 20).
 constexpr float kSkShared = 6.0f;
+// With whole waves after the cut tiles (sk_cut_tiles) the fix-ups pass under the main loops of the tiles after them, as long as those
+// are long enough.  A CTA's partial costs about 25 k-blocks to write and add (0.3 us each at 256 columns): 7100 and 2304 rows against
+// 3584 x 18944 gain 1244 -> 690 and 298 -> 234 us; with K = 3584 (2304 rows: 54 -> 71 us) the fix-ups are what is left.
+constexpr float kSkPartial = 25.0f;
+// The cost of the fix-ups of a launch, in k-blocks.
+static float sk_fix(int tiles, int k_blocks, int sms, float fix) {
+  const int cut = sk_cut_tiles(tiles, sms);
+  const float shared = static_cast<float>(sms) / static_cast<float>(std::max(cut, 1));
+  if (cut < tiles) {
+    const float own = kSkPartial * (1.f + shared);
+    return own < 0.5f * static_cast<float>(k_blocks) ? 0.25f * own : 1e6f;
+  }
+  return shared > kSkShared ? fix * shared / kSkShared : fix;
+}
 static bool stream_k_applies(int tiles, int k_blocks, int sms, float fix) {
   if (!stream_k_enabled() || tiles % sms == 0 || static_cast<long long>(tiles) * k_blocks < 2LL * sms) return false;
-  const float shared = static_cast<float>(sms) / static_cast<float>(tiles);
-  if (shared > kSkShared) fix *= shared / kSkShared;
   const float w = static_cast<float>(tiles) / static_cast<float>(sms);
   const float dp = static_cast<float>((tiles + sms - 1) / sms);
-  const float sk = w + fix / static_cast<float>(k_blocks);
+  const float sk = w + sk_fix(tiles, k_blocks, sms, fix) / static_cast<float>(k_blocks);
   return sk < 0.93f * dp;
 }
 // Relative duration of a launch with `tiles` tiles of relative cost `cost`: whole waves when tiles are dealt
 // round-robin, the exact share plus the fix-up when stream-K spreads the k-blocks evenly.
 static float launch_cost(int tiles, int k_blocks, int sms, float cost, float fix) {
   if (stream_k_applies(tiles, k_blocks, sms, fix))
-    return (static_cast<float>(tiles) / static_cast<float>(sms) + fix / static_cast<float>(k_blocks)) * cost;
+    return (static_cast<float>(tiles) / static_cast<float>(sms) + sk_fix(tiles, k_blocks, sms, fix) / static_cast<float>(k_blocks)) * cost;
   return static_cast<float>((tiles + sms - 1) / sms) * cost;
 }
 
@@ -748,6 +765,7 @@ static int launch_gemm(const void* A, const void* W, void* C, const void* bias, 
   uint32_t* sk_flags = nullptr;
   uint32_t sk_seq = 0;
   const int k_blocks = (K + kBK - 1) / kBK;
+  batch.raster = group_tab == nullptr && batch.count == 1 && static_cast<long long>(M) * K * 2 > kRasterBytes;
   if (group_tab == nullptr && stream_k_applies(tiles, k_blocks, sms, EPI == kEpiScatter ? kSkFixScatter : kSkFixPlain)) {
     SkWorkspace* w = sk_workspace(stream, sms);
     if (w != nullptr) {

@@ -47,6 +47,18 @@ def test_more_tiles_than_sms_in_ranges(m, n, k):
     ops.check_status()
 
 
+@pytest.mark.parametrize("m,n,k", [(2304, 1280, 18944), (300, 18952, 2048)])
+def test_whole_waves_and_a_cut_last_one(m, n, k):
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a = torch.randn(m, k, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(n, k, device="cuda", generator=g) * 0.05).bfloat16()
+    want = a.double() @ w.double().t()
+    for _ in range(2):
+        _check(ops.gemm(a, w, bn=64), want)
+        _check(ops.gemm(a, w), want)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("m", [1, 31, 32, 130])
 @pytest.mark.parametrize("inter,k", [(128, 64), (640, 200), (4096, 896)])
 def test_gated_products(m, inter, k):
