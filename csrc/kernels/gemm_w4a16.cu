@@ -23,8 +23,11 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "attention_common.cuh"
 #include "common.cuh"
+#include "gemm_rows.cuh"
 #include "ogb_kernels.h"
 
 namespace ogb {
@@ -366,6 +369,200 @@ gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint
   }
 }
 
+// ------------------------------------------------------------------------------------------
+// Few rows (M <= kRowsMaxM): the scheme of gemm_rows.cuh over int4 weights.  A decode step of a small model is bound by the chain
+// load -> dequantise -> multiply of a few CTAs, not by bytes: 64 rows against a 896 x 4864 projection left 14 CTAs to walk 76 k-blocks one
+// after the other (33 us for 2.3 MB).  Here 128 dequantised rows of W are the M side of the MMA, the activations its N side, and a
+// cluster shares the k-blocks of a tile (2 - 10 each at these sizes, whose loads are under way before the first is used).  The gated
+// form takes 128 gate and the matching 128 up rows per tile and stores silu(gate) * up: no [M, 2 N] round trip, no launch of its own.
+//   warp 0 TMA of the activations, warp 1 MMA, warps 2 .. 5 epilogue, warps 6 .. 13 dequantisers: a thread takes one 32-weight block
+//   per 128 rows of a k-block.
+// ------------------------------------------------------------------------------------------
+struct W4RowsParams {
+  const uint8_t* qw;
+  const void* scales;
+  const uint8_t* zp;
+  int kb32;                    // 32-weight blocks per row
+  int pair_step;               // rows of W between the two accumulators of a tile
+  int tile_rows;               // rows of W that tiles start in: a row index of a tile at or past it is not there
+};
+
+template <int TW, int EPI, bool SF32>
+__global__ void __launch_bounds__(kWThreads, 1)
+gemm_w4_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const RowsGemmParams p, const W4RowsParams wp, const ActArgs act) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  constexpr int kStageW = TW * kWTile * kWBK * 2;
+  const int stage_bytes = kStageW + p.mn * kWBK * 2;
+  const int ring_bytes = p.stages * stage_bytes;
+  RowsBars* bars = reinterpret_cast<RowsBars*>(smem + ring_bytes);
+  float* staging = reinterpret_cast<float*>(smem + ring_bytes + kRowsBarBytes);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int acc_cols, bufs;
+  uint32_t tmem_cols;
+  rows_tmem<TW>(p, acc_cols, bufs, tmem_cols);
+
+  // The dequantisers' first weights are requested before anything else: they depend on no barrier.
+  constexpr int kDepth = 4;                      // k-blocks ahead of their use
+  W4Unit ring[kDepth][TW];
+  const int t = static_cast<int>(threadIdx.x) - 6 * 32;
+  const int r_tile = t >> 1, half = t & 1;       // this thread's row of a tile and its 32-weight block of a k-block
+  RowsCursor cur(p);
+  auto fetch = [&](W4Unit (&un)[TW]) {
+    const int b = cur.kb * 2 + half;
+    const int row0 = cur.tile * kWTile * (EPI == kEpiSwiGLU ? 1 : TW) + r_tile;
+#pragma unroll
+    for (int w = 0; w < TW; ++w) {
+      const int n = row0 + w * wp.pair_step;
+      un[w].valid = cur.more && n < p.N && row0 < wp.tile_rows && b < wp.kb32;
+      const size_t row = un[w].valid ? n : 0;
+      const int bb = un[w].valid ? b : 0;
+      const size_t blk = row * wp.kb32 + bb;
+      un[w].q = __ldg(reinterpret_cast<const uint4*>(wp.qw) + blk);
+      if constexpr (SF32) un[w].s_raw = __float_as_uint(__ldg(static_cast<const float*>(wp.scales) + blk));
+      else un[w].s_raw = __ldg(static_cast<const unsigned short*>(wp.scales) + blk);
+      un[w].z_raw = 0x88u;
+      if (wp.zp != nullptr) un[w].z_raw = wp.zp[row * ((wp.kb32 + 1) / 2) + (bb >> 1)];
+    }
+    cur.step();
+  };
+  if (warp >= 6) {
+#pragma unroll
+    for (int d = 0; d < kDepth; ++d) fetch(ring[d]);
+  }
+  if (threadIdx.x == 0) tma_prefetch_desc(&tmap_a);
+  const uint32_t tmem_base = rows_setup(bars, p.stages, 1 + kWDequantWarps, tmem_cols);
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (RowsCursor c(p); c.more; c.step()) {
+        if (!mbar_wait(&bars->empty[stage], phase ^ 1)) { ok = false; break; }
+        mbar_expect_tx(&bars->full[stage], static_cast<uint32_t>(p.mn * kWBK * 2));
+        tma_load_2d(smem + stage * stage_bytes + kStageW, &tmap_a, &bars->full[stage], c.kb * kWBK, 0);
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
+      if (!ok) { atomicOr(p.status, kStatusWaitTimeout); bars->abort_flag = 1; }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0 && !rows_issue_mma<TW>(p, smem, stage_bytes, tmem_base, bufs, acc_cols, bars->full, bars->empty, bars->tmem_full, bars->tmem_empty)) {
+      atomicOr(p.status, kStatusWaitTimeout);
+      bars->abort_flag = 1;
+    }
+    __syncwarp();
+  } else if (warp < 6) {
+    if (p.splits == 0)
+      rows_epilogue<TW, EPI>(p, act, tmem_base, bufs, acc_cols, bars->tmem_full, bars->tmem_empty, &bars->abort_flag, staging, &bars->shared_last);
+  } else {
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    const RowsSegs all(p);
+    const int iters = static_cast<int>(all.it1 - all.it0);
+    for (int j0 = 0; ok && j0 < iters; j0 += kDepth) {
+#pragma unroll
+      for (int d = 0; d < kDepth; ++d) {
+        if (ok && j0 + d < iters) {
+          if (!__all_sync(0xffffffffu, mbar_wait(&bars->empty[stage], phase ^ 1))) {
+            ok = false;
+          } else {
+            tc_fence_after();              // the tensor core's reads of this slot are ordered before the stores below
+#pragma unroll
+            for (int w = 0; w < TW; ++w) {
+              uint8_t* sw = smem + stage * stage_bytes + w * (kWTile * kWBK * 2) + static_cast<uint32_t>(r_tile) * 128u;
+              const W4Unit& un = ring[d][w];
+              const uint32_t words[4] = {un.q.x, un.q.y, un.q.z, un.q.w};
+              const uint32_t z = half ? (un.z_raw >> 4) & 0xFu : un.z_raw & 0xFu;
+              const uint32_t zbits = 0x4300u | z;                       // bf16 128 + z, exact
+              const uint32_t zz_u = zbits | (zbits << 16);
+              uint32_t ss_u;
+              if constexpr (SF32) {
+                const __nv_bfloat162 tt = __float2bfloat162_rn(__uint_as_float(un.s_raw));
+                ss_u = *reinterpret_cast<const uint32_t*>(&tt);
+              } else {
+                ss_u = un.s_raw | (un.s_raw << 16);
+              }
+              if (!un.valid) ss_u = 0u;
+              const __nv_bfloat162 zz = *reinterpret_cast<const __nv_bfloat162*>(&zz_u);
+              const __nv_bfloat162 ss = *reinterpret_cast<const __nv_bfloat162*>(&ss_u);
+#pragma unroll
+              for (int wi = 0; wi < 4; ++wi) {
+                uint32_t o[4];
+                dequant_word(words[wi], zz, ss, o);
+                const uint32_t chunk = static_cast<uint32_t>(half * 4 + wi) ^ static_cast<uint32_t>(r_tile & 7);
+                *reinterpret_cast<uint4*>(sw + chunk * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+              }
+            }
+            fence_proxy_async_smem();      // the tensor core reads these bytes through the async proxy
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->full[stage]);
+            if (j0 + d + kDepth < iters) fetch(ring[d]);
+            if (++stage == p.stages) { stage = 0; phase ^= 1; }
+          }
+        }
+      }
+    }
+    if (!ok && lane == 0) { atomicOr(p.status, kStatusWaitTimeout); bars->abort_flag = 1; }
+    __syncwarp();
+  }
+  if (p.splits > 0) rows_finish_cluster<TW, EPI>(p, act, tmem_base, acc_cols, bars->tmem_full, &bars->abort_flag, smem, ring_bytes);
+  rows_teardown(bars, tmem_base, tmem_cols);
+}
+
+template <int TW, int EPI, bool SF32>
+static int launch_w4_rows_one(const void* x, int K, int ldx, RowsGemmParams p, W4RowsParams wp, cudaStream_t stream) {
+  auto kernel = gemm_w4_rows_kernel<TW, EPI, SF32>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    OGB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmemMax));
+    attr_set = true;
+  }
+  const int sms = ogb_num_sms();
+  const int stage_bytes = TW * kWTile * kWBK * 2 + p.mn * kWBK * 2;
+  p.n_tiles = (wp.tile_rows + kWTile - 1) / kWTile;
+  int grid, smem;
+  if (p.n_tiles > sms) {
+    if (p.M > kRowsRangesM) return kRowsDeclined;
+    p.splits = 0;
+    grid = sms;
+    p.stages = std::min(kRowsMaxStages, (kRowsSmemMax - kRowsBarBytes - TW * kRowsStage) / stage_bytes);
+    smem = p.stages * stage_bytes + kRowsBarBytes + TW * kRowsStage;
+    void* ws = rows_workspace(stream, grid, TW, p.mn);
+    if (ws == nullptr) return kRowsDeclined;
+    p.counters = static_cast<unsigned int*>(ws);
+    p.ws = reinterpret_cast<float*>(static_cast<char*>(ws) + rows_counter_bytes(sms));
+  } else {
+    p.stages = std::min(kRowsMaxStages, (kRowsSmemMax - kRowsBarBytes) / stage_bytes);
+    smem = p.stages * stage_bytes + kRowsBarBytes;
+    p.splits = rows_pick_splits(kernel, kWThreads, smem, p.n_tiles, p.k_blocks);
+    grid = p.n_tiles * p.splits;
+  }
+  CUtensorMap ta;
+  const int rc = make_tmap_bf16_2d(&ta, x, p.M, K, ldx, p.mn, kWBK);
+  if (rc != 0) return rc;
+  return rows_launch(kernel, grid, kWThreads, smem, p.splits, stream, ta, p, wp, ActArgs());
+}
+
+static int launch_w4_rows(const void* x, const void* qweight, const void* scales, const void* zp, const void* bias, void* out, int M, int N, int K,
+                          int ldx, int ldc, bool scales_f32, bool gated, int* status, cudaStream_t stream) {
+  RowsGemmParams p{};
+  W4RowsParams wp{};
+  p.mn = (M + 15) / 16 * 16;
+  p.k_blocks = (K + kWBK - 1) / kWBK;
+  p.C = static_cast<__nv_bfloat16*>(out);
+  p.bias = static_cast<const __nv_bfloat16*>(bias != nullptr ? bias : qweight);       // N * K / 2 bytes, K >= 32
+  p.has_bias = bias != nullptr;
+  p.M = M; p.N = N; p.ldc = ldc; p.status = status;
+  wp.qw = static_cast<const uint8_t*>(qweight); wp.scales = scales; wp.zp = static_cast<const uint8_t*>(zp);
+  wp.kb32 = K / 32;
+  wp.pair_step = gated ? N / 2 : kWTile;
+  wp.tile_rows = gated ? N / 2 : N;
+  if (gated) return scales_f32 ? launch_w4_rows_one<2, kEpiSwiGLU, true>(x, K, ldx, p, wp, stream) : launch_w4_rows_one<2, kEpiSwiGLU, false>(x, K, ldx, p, wp, stream);
+  return scales_f32 ? launch_w4_rows_one<1, kEpiNone, true>(x, K, ldx, p, wp, stream) : launch_w4_rows_one<1, kEpiNone, false>(x, K, ldx, p, wp, stream);
+}
+
 template <int MT, bool SF32, int TN>
 static int launch_w4a16_gemm(const void* x, const void* qweight, const void* scales, const void* zp, const void* bias, void* out,
                              int M, int N, int K, int ldx, int ldc, int* status, cudaStream_t stream) {
@@ -399,6 +596,10 @@ extern "C" int ogb_w4a16_gemm(const void* x, const void* qweight, const void* sc
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((K % 32) != 0 || (ldx % 8) != 0 || (ldc % 8) != 0) return -3;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(qweight)) & 15) return -4;
+  if (M <= kRowsMaxM) {
+    const int rc = launch_w4_rows(x, qweight, scales, zp, bias, out, M, N, K, ldx, ldc, scales_f32 != 0, false, status, stream);
+    if (rc != kRowsDeclined) return rc;
+  }
   // 64-column W tiles when 128-column ones would occupy at most half of the SMs: the dequantisers of a CTA, not its
   // tensor core, set the pace, so twice the CTAs over half the rows each is close to twice as fast (down and o
   // projections at decode-sized M).
@@ -413,4 +614,15 @@ extern "C" int ogb_w4a16_gemm(const void* x, const void* qweight, const void* sc
   if (narrow) return scales_f32 ? OGB_W4_LAUNCH(1, true, 64) : OGB_W4_LAUNCH(1, false, 64);
   return scales_f32 ? OGB_W4_LAUNCH(1, true, 128) : OGB_W4_LAUNCH(1, false, 128);
 #undef OGB_W4_LAUNCH
+}
+
+// out[M, N / 2] = silu(gate) * up of a projection whose first N / 2 rows are the gate's and the others the up projection's; arguments as
+// above, without a bias.  M at most 256.  -11: not here (a capture outside a step has no workspace).
+extern "C" int ogb_w4a16_gated(const void* x, const void* qweight, const void* scales, const void* zp, void* out, int M, int N, int K, int ldx, int ldc,
+                               int scales_f32, int* status, void* stream_) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (M > kRowsMaxM || (N % 2) != 0 || (K % 32) != 0 || (ldx % 8) != 0 || (ldc % 8) != 0) return -3;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(qweight)) & 15) return -4;
+  const int rc = launch_w4_rows(x, qweight, scales, zp, nullptr, out, M, N, K, ldx, ldc, scales_f32 != 0, true, status, static_cast<cudaStream_t>(stream_));
+  return rc == kRowsDeclined ? -11 : rc;
 }

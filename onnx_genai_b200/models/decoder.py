@@ -601,12 +601,14 @@ class DecoderModel:
                 self._norm(x, lw.ln2, pending, h)
                 inter = lw.quant["gate"].n
                 gu = self.gate_up[:t, : 2 * inter]
-                if lw.quant.get("gate_up") is not None:
-                    lw.quant["gate_up"](h, out=gu)
-                else:
-                    lw.quant["gate"](h, out=gu[:, :inter])
-                    lw.quant["up"](h, out=gu[:, inter:])
-                act = ops.silu_mul(gu, out=self.act_q[:t]) if x.is_cuda else ops.silu_mul(gu)
+                act = self.act_q[:t]
+                if lw.quant.get("gate_up") is None or not lw.quant["gate_up"].gated(h, act):
+                    if lw.quant.get("gate_up") is not None:
+                        lw.quant["gate_up"](h, out=gu)
+                    else:
+                        lw.quant["gate"](h, out=gu[:, :inter])
+                        lw.quant["up"](h, out=gu[:, inter:])
+                    act = ops.silu_mul(gu, out=act) if x.is_cuda else ops.silu_mul(gu)
                 pending = lw.quant["down"](act, out=self.partial[:t])
                 continue
             pending = self._row_parallel(attn, lw.o_w, x, 0)
