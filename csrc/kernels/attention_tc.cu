@@ -180,7 +180,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
   if (rows <= 0 || ctx <= 0) return;
   // A tile with few rows takes several query heads of its KV head: 1 << row_bits tile rows per head.  The later turn of a
   // conversation -- at most 16 new tokens against a long context -- then reads the context once for 8 heads instead of 8 times
-  // with 16 of 128 rows in use (256 sequences of 614 tokens and 16 rows each, 28 heads over 4: 895 -> 197 us).
+  // with 16 of 128 rows in use (256 sequences of 614 tokens and 16 rows each, 28 heads over 4: 895 -> 177 us).
   const int row_bits = CHUNKED || rows > 64 ? 7 : rows > 32 ? 6 : rows > 16 ? 5 : 4;
   const int heads_here = min(kFaBM >> row_bits, p.group - head % p.group);
   if ((head % p.group) & ((kFaBM >> row_bits) - 1)) return;        // served with an earlier head of the group
@@ -212,6 +212,15 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
   if (warp == 2) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
     tmem_relinquish();
+  }
+  if (row_bits != 7) {
+    // query rows that no head fills: whatever they held would send blocks down the masked path (21 -> 28 us for 9 rows of 777 tokens)
+    const int first = heads_here << row_bits;
+    for (int i = threadIdx.x; i < (kFaBM - first) * Cfg::kHalvesK * 8; i += kFaThreads) {
+      const int h = i / ((kFaBM - first) * 8), r = i % ((kFaBM - first) * 8);
+      *reinterpret_cast<uint4*>(sQ + h * Cfg::kHalfStrideQ + first * 128 + r * 16) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    fence_proxy_async_smem();
   }
   tc_fence_before();
   __syncthreads();
