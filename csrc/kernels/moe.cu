@@ -189,6 +189,64 @@ __global__ void moe_assign_kernel(const int* __restrict__ topk_ids, const int* _
   route_pos[i] = pos;
 }
 
+// All of the above in one CTA, for few routes: a decode step's 256 routes paid four launches (12 us) for a microsecond's work.
+constexpr int kPermuteOneRoutes = 4096;      // above: the counters' atomics of one SM take longer than the launches
+__global__ void __launch_bounds__(1024) moe_permute_one_kernel(const int* __restrict__ topk_ids, int* __restrict__ offsets, int* __restrict__ sorted_route,
+                                                               int* __restrict__ route_pos, int* __restrict__ tile_tab, int* __restrict__ meta, int routes,
+                                                               int e0, int experts, int max_mtiles) {
+  __shared__ int s_cnt[kMaxExperts], s_cur[kMaxExperts];
+  for (int e = threadIdx.x; e < kMaxExperts; e += blockDim.x) s_cnt[e] = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < routes; i += blockDim.x) {
+    const int e = topk_ids[i] - e0;
+    if (e >= 0 && e < experts) atomicAdd(&s_cnt[e], 1);
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    // a lane's eight neighbouring experts, then a scan over the lanes: rows in the low half of a word, 128-row tiles in the high one
+    constexpr int kPer = kMaxExperts / 32;
+    const int lane = threadIdx.x;
+    unsigned long long sum = 0, own[kPer];
+#pragma unroll
+    for (int x = 0; x < kPer; ++x) {
+      const int c = s_cnt[lane * kPer + x];
+      own[x] = sum;
+      sum += static_cast<unsigned long long>(c) | (static_cast<unsigned long long>((c + 127) / 128) << 32);
+    }
+    unsigned long long incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long n = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += n;
+    }
+#pragma unroll
+    for (int x = 0; x < kPer; ++x) {
+      const int e = lane * kPer + x;
+      const unsigned long long at = incl - sum + own[x];
+      const int row = static_cast<int>(at & 0xffffffffu), end = row + s_cnt[e];
+      s_cur[e] = row;
+      if (e < experts) {
+        offsets[e] = row;
+        int t = static_cast<int>(at >> 32);
+        for (int r = row; r < end && t < max_mtiles; r += 128, ++t) reinterpret_cast<int4*>(tile_tab)[t] = make_int4(e, r, end, 0);
+      }
+    }
+    if (lane == 31) {
+      offsets[experts] = static_cast<int>(incl & 0xffffffffu);
+      meta[0] = min(static_cast<int>(incl >> 32), max_mtiles);
+      meta[1] = static_cast<int>(incl & 0xffffffffu);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < routes; i += blockDim.x) {
+    const int e = topk_ids[i] - e0;
+    const bool mine = e >= 0 && e < experts;
+    const int pos = mine ? atomicAdd(&s_cur[e], 1) : -1;
+    if (mine) sorted_route[pos] = i;
+    route_pos[i] = pos;
+  }
+}
+
 __global__ void moe_gather_rows_kernel(const uint4* __restrict__ x, const int* __restrict__ sorted_route, const int* __restrict__ meta,
                                        uint4* __restrict__ xs, int k, int vecs) {
   const int pos = blockIdx.x;
@@ -199,34 +257,42 @@ __global__ void moe_gather_rows_kernel(const uint4* __restrict__ x, const int* _
   for (int i = threadIdx.x; i < vecs; i += blockDim.x) dst[i] = src[i];
 }
 
+// The rows of eight routes are requested together (one after the other, with each route's place looked up in front of it, a token of eight
+// routes took 11 us).
 __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ ys, const int* __restrict__ route_pos,
                                    const float* __restrict__ topk_w, __nv_bfloat16* __restrict__ out, int k, int hidden,
                                    int accumulate) {
   const int t = blockIdx.x;
-  for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) {
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (accumulate) {
-      const uint4 v = reinterpret_cast<const uint4*>(out + static_cast<size_t>(t) * hidden)[i];
-      float2 f;
-      f = unpack_bf16(v.x); acc[0] = f.x; acc[1] = f.y;
-      f = unpack_bf16(v.y); acc[2] = f.x; acc[3] = f.y;
-      f = unpack_bf16(v.z); acc[4] = f.x; acc[5] = f.y;
-      f = unpack_bf16(v.w); acc[6] = f.x; acc[7] = f.y;
+  const int i = blockIdx.y * blockDim.x + threadIdx.x;
+  if (i >= hidden / 8) return;
+  uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(t) * hidden) + i;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  auto add = [&](const uint4& v, float w) {
+    float2 f;
+    f = unpack_bf16(v.x); acc[0] += w * f.x; acc[1] += w * f.y;
+    f = unpack_bf16(v.y); acc[2] += w * f.x; acc[3] += w * f.y;
+    f = unpack_bf16(v.z); acc[4] += w * f.x; acc[5] += w * f.y;
+    f = unpack_bf16(v.w); acc[6] += w * f.x; acc[7] += w * f.y;
+  };
+  if (accumulate) add(*dst, 1.f);
+  for (int j0 = 0; j0 < k; j0 += 8) {
+    int pos[8];
+    float w[8];
+    uint4 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const size_t at = static_cast<size_t>(t) * k + min(j0 + j, k - 1);
+      pos[j] = j0 + j < k ? route_pos[at] : -1;      // -1: the route's expert lives on another rank
+      w[j] = topk_w[at];
     }
-    for (int j = 0; j < k; ++j) {
-      const int pos = route_pos[static_cast<size_t>(t) * k + j];
-      if (pos < 0) continue;   // the route's expert lives on another rank
-      const float w = topk_w[static_cast<size_t>(t) * k + j];
-      const uint4 v = reinterpret_cast<const uint4*>(ys + static_cast<size_t>(pos) * hidden)[i];
-      float2 f;
-      f = unpack_bf16(v.x); acc[0] += w * f.x; acc[1] += w * f.y;
-      f = unpack_bf16(v.y); acc[2] += w * f.x; acc[3] += w * f.y;
-      f = unpack_bf16(v.z); acc[4] += w * f.x; acc[5] += w * f.y;
-      f = unpack_bf16(v.w); acc[6] += w * f.x; acc[7] += w * f.y;
-    }
-    reinterpret_cast<uint4*>(out + static_cast<size_t>(t) * hidden)[i] =
-        make_uint4(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]), pack_bf16(acc[4], acc[5]), pack_bf16(acc[6], acc[7]));
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (pos[j] >= 0) v[j] = reinterpret_cast<const uint4*>(ys + static_cast<size_t>(pos[j]) * hidden)[i];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (pos[j] >= 0) add(v[j], w[j]);
   }
+  *dst = make_uint4(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]), pack_bf16(acc[4], acc[5]), pack_bf16(acc[6], acc[7]));
 }
 
 }  // namespace ogb
@@ -267,6 +333,11 @@ extern "C" int ogb_moe_permute(const int* topk_ids, int* counts, int* offsets, i
   if (experts > kMaxExperts) return -3;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int routes = tokens * k;
+  if (routes <= kPermuteOneRoutes && (reinterpret_cast<uintptr_t>(tile_tab) & 15) == 0) {
+    moe_permute_one_kernel<<<1, routes <= 256 ? 256 : 1024, 0, st>>>(topk_ids, offsets, sorted_route, route_pos, tile_tab, meta, routes, e0, experts,
+                                                                     max_mtiles);
+    return static_cast<int>(cudaGetLastError());
+  }
   OGB_CUDA_CHECK(cudaMemsetAsync(counts, 0, sizeof(int) * experts, st));
   moe_count_kernel<<<(routes + 255) / 256, 256, 0, st>>>(topk_ids, counts, routes, e0, experts);
   moe_plan_kernel<<<1, 256, 0, st>>>(counts, offsets, cursor, tile_tab, meta, experts, max_mtiles);
@@ -297,7 +368,7 @@ extern "C" int ogb_moe_combine(const void* ys, const int* route_pos, const float
                                int hidden, int accumulate, void* stream) {
   if (tokens <= 0) return 0;
   if (hidden % 8) return -3;
-  moe_combine_kernel<<<tokens, 128, 0, static_cast<cudaStream_t>(stream)>>>(
+  moe_combine_kernel<<<dim3(tokens, (hidden / 8 + 127) / 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(ys), route_pos, topk_w, static_cast<__nv_bfloat16*>(out), k, hidden, accumulate);
   return static_cast<int>(cudaGetLastError());
 }

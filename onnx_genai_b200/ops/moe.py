@@ -46,7 +46,7 @@ def moe_experts(h, router_logits, expert_gate_up, expert_down, ws: MoEWorkspace,
                 accumulate=True):
     """out (+)= sum over this rank's experts of w * down(swiglu(gate_up(h))).
 
-    router_logits [T, E_total] bf16; expert_gate_up [E_local, 2I, H] packed per expert with half-width
+    router_logits [T, E_total] bf16 or fp32; expert_gate_up [E_local, 2I, H] packed per expert with half-width
     ``half``; expert_down [E_local, H, I]; e0 = first global expert id held locally.
     """
     t, hidden = h.shape
@@ -70,8 +70,12 @@ def moe_experts(h, router_logits, expert_gate_up, expert_down, ws: MoEWorkspace,
     st = status_word(h.device).data_ptr()
     s = _stream()
     with timed_region("moe_route_permute"):
-        rc = lib.ogb_moe_route_topk(router_logits.data_ptr(), ws.topk_ids.data_ptr(), ws.topk_w.data_ptr(), t, e_total, k,
-                                    int(renormalize), router_logits.stride(0), s)
+        if router_logits.dtype == torch.float32:
+            rc = lib.ogb_moe_route_grouped(router_logits.data_ptr(), 0, ws.topk_ids.data_ptr(), ws.topk_w.data_ptr(), t, e_total, k, int(renormalize),
+                                           router_logits.stride(0), 1, 1, 0, 1, s)
+        else:
+            rc = lib.ogb_moe_route_topk(router_logits.data_ptr(), ws.topk_ids.data_ptr(), ws.topk_w.data_ptr(), t, e_total, k,
+                                        int(renormalize), router_logits.stride(0), s)
         _native.check(rc, "ogb_moe_route_topk")
         rc = lib.ogb_moe_permute(ws.topk_ids.data_ptr(), ws.counts.data_ptr(), ws.offsets.data_ptr(), ws.cursor.data_ptr(),
                                  ws.sorted_route.data_ptr(), ws.route_pos.data_ptr(), ws.tile_tab.data_ptr(), ws.meta.data_ptr(),
