@@ -46,6 +46,7 @@ __global__ void __launch_bounds__((ROWS / 16 + 1) * 32, 2) paged_prefill_kernel(
   uint64_t* empty_bar = full_bar + Cfg::kStages;
 
   const int tile = blockIdx.x / kSub;
+  pdl_trigger();
   if (tile >= p.num_tiles) return;
   const int head = blockIdx.y;
   const int kvh = head / p.group;
@@ -67,10 +68,11 @@ __global__ void __launch_bounds__((ROWS / 16 + 1) * 32, 2) paged_prefill_kernel(
     tma_prefetch_desc(&kv_map);
   }
   __syncthreads();
+  pdl_wait();
 
   if (warp == kWarps) {
     if (lane == 0) {
-      if (!attn_produce<Cfg>(&kv_map, p, stages, full_bar, empty_bar, seq, kvh, ctx, blocks, 0, blocks.count))
+      if (!attn_produce<Cfg>(&kv_map, p, stages, full_bar, empty_bar, seq, kvh, ctx, blocks, 0, blocks.count, 0))
         atomicOr(p.status, kStatusWaitTimeout);
     }
     return;
@@ -224,6 +226,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) paged_decode_kernel(const __g
   uint64_t* empty_bar = full_bar + Cfg::kStages;
   float* sm_ml = reinterpret_cast<float*>(empty_bar + Cfg::kStages);  // [4 warps][16 rows][2]
 
+  pdl_trigger();
   const int seq = blockIdx.x / p.num_splits;
   const int split = blockIdx.x % p.num_splits;
   const int kvh = blockIdx.y;
@@ -242,6 +245,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) paged_decode_kernel(const __g
   const int kv_lo = blocks.kv_lo;
   if (b_begin >= b_end) {
     // nothing to do for this split (or an inactive row): publish an empty partial
+    pdl_wait();
     if (p.num_splits > 1 && ctx > 0) {
       for (int idx = threadIdx.x; idx < G * D; idx += blockDim.x) {
         const int r = idx / D, d = idx % D;
@@ -262,12 +266,13 @@ __global__ void __launch_bounds__(kAttnThreads, 2) paged_decode_kernel(const __g
 
   if (warp == 4) {
     if (lane == 0) {
-      if (!attn_produce<Cfg>(&kv_map, p, stages, full_bar, empty_bar, seq, kvh, ctx, blocks, b_begin, b_end))
+      if (!attn_produce<Cfg>(&kv_map, p, stages, full_bar, empty_bar, seq, kvh, ctx, blocks, b_begin, b_end, ctx - 1))
         atomicOr(p.status, kStatusWaitTimeout);
     }
     return;
   }
 
+  pdl_wait();
   {
     const __nv_bfloat16* qsrc = p.q + static_cast<size_t>(seq) * p.q_stride + kvh * G * D;
     for (int idx = threadIdx.x; idx < 16 * (D / 8); idx += 128) {
@@ -415,6 +420,10 @@ __global__ void __launch_bounds__(kAttnThreads, 2) paged_decode_kernel(const __g
 __global__ void paged_decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                           const int* __restrict__ ctx_len, __nv_bfloat16* __restrict__ out, int hq, int D,
                                           int num_splits, int o_stride) {
+  pdl_trigger();
+  pdl_wait();
+  part_o = after_wait(part_o);
+  part_ml = after_wait(part_ml);
   const int seq = blockIdx.x, head = blockIdx.y;
   if (ctx_len[seq] <= 0) return;
   const size_t base = (static_cast<size_t>(seq) * hq + head) * num_splits;
@@ -473,8 +482,7 @@ static int launch_prefill_rows(const CUtensorMap& map, const AttnParams& p, cuda
     attr_set = true;
   }
   dim3 grid(p.num_tiles * (64 / ROWS), p.hq);
-  paged_prefill_kernel<D, ROWS><<<grid, (ROWS / 16 + 1) * 32, Cfg::kSmemBytes, stream>>>(map, p);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_overlapped(paged_prefill_kernel<D, ROWS>, grid, dim3((ROWS / 16 + 1) * 32), Cfg::kSmemBytes, stream, map, p));
 }
 
 template <int D>
@@ -496,13 +504,12 @@ static int launch_decode(const CUtensorMap& map, const AttnParams& p, cudaStream
     attr_set = true;
   }
   dim3 grid(p.num_seqs * p.num_splits, p.hkv);
-  paged_decode_kernel<D><<<grid, kAttnThreads, Cfg::kSmemBytes, stream>>>(map, p);
-  int rc = static_cast<int>(cudaGetLastError());
+  int rc = static_cast<int>(launch_overlapped(paged_decode_kernel<D>, grid, dim3(kAttnThreads), Cfg::kSmemBytes, stream, map, p));
   if (rc != 0) return rc;
   if (p.num_splits > 1) {
     dim3 mgrid(p.num_seqs, p.hq);
-    paged_decode_merge_kernel<<<mgrid, D, 0, stream>>>(p.part_o, p.part_ml, p.ctx_len, p.out, p.hq, D, p.num_splits, p.o_stride);
-    rc = static_cast<int>(cudaGetLastError());
+    rc = static_cast<int>(launch_overlapped(paged_decode_merge_kernel, mgrid, dim3(D), 0, stream, p.part_o, p.part_ml, p.ctx_len, p.out, p.hq, D,
+                                            p.num_splits, p.o_stride));
   }
   return rc;
 }

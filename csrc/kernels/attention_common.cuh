@@ -123,13 +123,19 @@ OGB_DEVICE KvBlocks make_kv_blocks(int window, int sink, int kv_lo, int kv_end, 
 // Producer: stream logical blocks [j_begin, j_end) of one sequence / kv head into the ring.
 template <class Cfg>
 OGB_DEVICE bool attn_produce(const CUtensorMap* kv_map, const AttnParams& p, uint8_t* stages, uint64_t* full_bar,
-                             uint64_t* empty_bar, int seq, int kvh, int ctx, const KvBlocks& blocks, int j_begin, int j_end) {
+                             uint64_t* empty_bar, int seq, int kvh, int ctx, const KvBlocks& blocks, int j_begin, int j_end, int fresh) {
   const int n_pages = (ctx + kPageTokens - 1) / kPageTokens;
   const int* table = p.page_table + static_cast<size_t>(seq) * p.max_pages;
   int stage = 0;
   uint32_t phase = 0;
+  // keys from `fresh` on are written by the kernels right before this one; earlier ones are there already
+  bool waited = false;
   for (int j = j_begin; j < j_end; ++j) {
     const int b = blocks.phys(j);
+    if (!waited && (b + 1) * kKvBlock > fresh) {
+      pdl_wait();
+      waited = true;
+    }
     if (!mbar_wait(&empty_bar[stage], phase ^ 1)) return false;
     uint8_t* sk = stages + stage * Cfg::kStageBytes;
     uint8_t* sv = sk + Cfg::kTileBytes;

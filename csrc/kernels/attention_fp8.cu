@@ -114,12 +114,17 @@ OGB_DEVICE void expand_page(const uint8_t* raw, uint8_t* work, int tid, int nthr
 }
 
 OGB_DEVICE bool fp8_produce(const CUtensorMap* kv_map, const AttnParams& p, uint8_t* stages, uint64_t* full_bar,
-                            uint64_t* empty_bar, int nstages, int seq, int kvh, int ctx, int b_begin, int b_end, int kv_lo) {
+                            uint64_t* empty_bar, int nstages, int seq, int kvh, int ctx, int b_begin, int b_end, int kv_lo, int fresh) {
   const int n_pages = (ctx + kPageTokens - 1) / kPageTokens;
   const int* table = p.page_table + static_cast<size_t>(seq) * p.max_pages;
   int stage = 0;
   uint32_t phase = 0;
+  bool waited = false;                   // keys from `fresh` on are written by the kernels right before this one
   for (int b = b_begin; b < b_end; ++b) {
+    if (!waited && (b + 1) * kKvBlock > fresh) {
+      pdl_wait();
+      waited = true;
+    }
     int64_t page_of_slot[4];             // read ahead of the wait for the slot
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -167,6 +172,7 @@ __global__ void __launch_bounds__(kAttnThreads) paged_decode_fp8_kernel(const __
   uint64_t* empty_bar = full_bar + kDecStages;
   float* sm_ml = reinterpret_cast<float*>(empty_bar + kDecStages);
 
+  pdl_trigger();
   const int seq = blockIdx.x / p.num_splits, split = blockIdx.x % p.num_splits, kvh = blockIdx.y;
   const int G = p.group;
   const int ctx = p.ctx_len[seq];
@@ -182,6 +188,7 @@ __global__ void __launch_bounds__(kAttnThreads) paged_decode_fp8_kernel(const __
     b_end = min(b_begin + per, last);
   }
   if (b_begin >= b_end) {
+    pdl_wait();
     if (p.num_splits > 1 && ctx > 0) {
       for (int idx = threadIdx.x; idx < G * kD; idx += blockDim.x) {
         const int r = idx / kD, d = idx % kD;
@@ -199,10 +206,11 @@ __global__ void __launch_bounds__(kAttnThreads) paged_decode_fp8_kernel(const __
   }
   __syncthreads();
   if (warp == 4) {
-    if (lane == 0 && !fp8_produce(&kv_map, p, stages, full_bar, empty_bar, kDecStages, seq, kvh, ctx, b_begin, b_end, kv_lo))
+    if (lane == 0 && !fp8_produce(&kv_map, p, stages, full_bar, empty_bar, kDecStages, seq, kvh, ctx, b_begin, b_end, kv_lo, ctx - 1))
       atomicOr(p.status, kStatusWaitTimeout);
     return;
   }
+  pdl_wait();
   {
     const __nv_bfloat16* qsrc = p.q + static_cast<size_t>(seq) * p.q_stride + kvh * G * kD;
     for (int idx = threadIdx.x; idx < 16 * (kD / 8); idx += 128) {
@@ -357,6 +365,10 @@ __global__ void paged_decode_fp8_merge_kernel(const float* __restrict__ part_o, 
                                               const int* __restrict__ ctx_len, __nv_bfloat16* __restrict__ out, int hq,
                                               int num_splits, int o_stride) {
   const int seq = blockIdx.x, head = blockIdx.y;
+  pdl_trigger();
+  pdl_wait();
+  part_o = after_wait(part_o);
+  part_ml = after_wait(part_ml);
   if (ctx_len[seq] <= 0) return;
   const size_t base = (static_cast<size_t>(seq) * hq + head) * num_splits;
   float mx = -INFINITY;
@@ -451,7 +463,12 @@ OGB_DEVICE bool fp8_produce_wide(const CUtensorMap* kv_map, const AttnParams& p,
   const int* table = p.page_table + static_cast<size_t>(seq) * p.max_pages;
   int stage = 0;
   uint32_t phase = 0;
+  bool waited = false;                   // the newest key, and its page's scale, come from the kernels right before this one
   for (int b = b_begin; b < b_end; ++b) {
+    if (!waited && (b + 1) * kMmaKeys >= ctx) {
+      pdl_wait();
+      waited = true;
+    }
     const int n_load = min(kMmaPages, ((n_pages - b * kMmaPages + 1) >> 1) << 1);
     int64_t page = 0;
     if (lane < n_load) {
@@ -488,6 +505,7 @@ __global__ void __maxnreg__(168) paged_decode_e4m3_mma_kernel(const __grid_const
   float* sm_ml = reinterpret_cast<float*>(empty_bar + kMmaStages);   // [4 warps][8 rows][2]
   float* stage_scales = sm_ml + 4 * 8 * 2;                           // [stages][8 pages][K, V]
 
+  pdl_trigger();
   const int seq = blockIdx.x / p.num_splits, split = blockIdx.x % p.num_splits, kvh = blockIdx.y;
   const int G = p.group;
   const int ctx = p.ctx_len[seq];
@@ -503,6 +521,7 @@ __global__ void __maxnreg__(168) paged_decode_e4m3_mma_kernel(const __grid_const
     b_end = min(b_begin + per, last);
   }
   if (b_begin >= b_end) {
+    pdl_wait();
     if (p.num_splits > 1 && ctx > 0) {
       for (int idx = threadIdx.x; idx < G * kD; idx += blockDim.x) {
         const int r = idx / kD, d = idx % kD;
@@ -524,6 +543,7 @@ __global__ void __maxnreg__(168) paged_decode_e4m3_mma_kernel(const __grid_const
       atomicOr(p.status, kStatusWaitTimeout);
     return;
   }
+  pdl_wait();
   const int g = lane >> 2, q = lane & 3;
 
   // query fragments: row g = hi part, row g + 8 = lo part of head kvh * G + g; k runs over the head dimension
@@ -756,7 +776,7 @@ __global__ void __launch_bounds__(kAttnThreads) paged_prefill_fp8_kernel(const _
   }
   __syncthreads();
   if (warp == 4) {
-    if (lane == 0 && !fp8_produce(&kv_map, p, stages, full_bar, empty_bar, kPreStages, seq, kvh, ctx, b_begin, b_end, kv_lo))
+    if (lane == 0 && !fp8_produce(&kv_map, p, stages, full_bar, empty_bar, kPreStages, seq, kvh, ctx, b_begin, b_end, kv_lo, 0))
       atomicOr(p.status, kStatusWaitTimeout);
     if (splits > 1) {
       __syncwarp();
@@ -1018,14 +1038,14 @@ static int launch_decode_q(const void* q, void* out, const void* pool, const flo
       OGB_CUDA_CHECK(cudaFuncSetAttribute(paged_decode_e4m3_mma_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
       mma_attr_set = true;
     }
-    paged_decode_e4m3_mma_kernel<<<dim3(num_seqs * num_splits, hkv), kAttnThreads, kMmaSmem, st>>>(map, p);
+    OGB_CUDA_CHECK(launch_overlapped(paged_decode_e4m3_mma_kernel, dim3(num_seqs * num_splits, hkv), dim3(kAttnThreads), kMmaSmem, st, map, p));
   } else {
-    paged_decode_fp8_kernel<<<dim3(num_seqs * num_splits, hkv), kAttnThreads, kDecSmem, st>>>(map, p);
+    OGB_CUDA_CHECK(launch_overlapped(paged_decode_fp8_kernel, dim3(num_seqs * num_splits, hkv), dim3(kAttnThreads), kDecSmem, st, map, p));
   }
   rc = static_cast<int>(cudaGetLastError());
   if (rc == 0 && num_splits > 1) {
-    paged_decode_fp8_merge_kernel<<<dim3(num_seqs, hq), kD, 0, st>>>(part_o, part_ml, ctx_len, p.out, hq, num_splits, o_stride);
-    rc = static_cast<int>(cudaGetLastError());
+    rc = static_cast<int>(launch_overlapped(paged_decode_fp8_merge_kernel, dim3(num_seqs, hq), dim3(kD), 0, st, part_o, part_ml, ctx_len, p.out, hq,
+                                            num_splits, o_stride));
   }
   return rc;
 }

@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(kTcThreads) paged_decode_e4m3_tc_kernel(const 
     b_end = min(b_begin + per, last);
   }
   if (b_begin >= b_end) {
+    pdl_wait();
     if (p.num_splits > 1 && ctx > 0) {
       for (int idx = threadIdx.x; idx < G * kTcD; idx += blockDim.x) {
         const int r = idx / kTcD, d = idx % kTcD;
@@ -200,6 +201,7 @@ __global__ void __launch_bounds__(kTcThreads) paged_decode_e4m3_tc_kernel(const 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sh.tmem_base;
+  pdl_trigger();
   volatile int* abort_flag = &sh.abort_flag;
   const bool dbg_cta = p.dbg != nullptr && static_cast<int>(blockIdx.x) == p.dbg_tile && blockIdx.y == 0;
   TcStamp stamp{(dbg_cta && lane == 0 && (warp == 0 || warp == 1 || warp == 4)) ? p.dbg : nullptr, 0};
@@ -213,8 +215,13 @@ __global__ void __launch_bounds__(kTcThreads) paged_decode_e4m3_tc_kernel(const 
     uint64_t* empty = side ? sh.v_empty : sh.k_empty;
     const int n_pages = (ctx + kPageTokens - 1) / kPageTokens;
     const int* table = p.page_table + static_cast<size_t>(seq) * p.max_pages;
+    bool waited = false;     // the newest key, and its page's scales, come from the kernels right before this one
     for (int i = 0; i < n_blocks; ++i) {
       const int b = b_begin + i, s = i % kTcStages;
+      if (!waited && (b + 1) * kTcKeys >= ctx) {
+        pdl_wait();
+        waited = true;
+      }
       // K pages past the context are skipped (their keys are masked); V is always filled: masked probabilities are
       // zeros, and a zero must meet finite bytes.
       const int n_load = side ? kTcPages : min(kTcPages, n_pages - b * kTcPages);
@@ -296,6 +303,7 @@ __global__ void __launch_bounds__(kTcThreads) paged_decode_e4m3_tc_kernel(const 
     const int quarter = warp & 3;
     const int t = 32 * quarter + lane;
     const uint32_t lane_base = tmem + (static_cast<uint32_t>(32 * quarter) << 16);
+    pdl_wait();
     {
       // Qhl tile: thread (r, c) writes 16 bytes of row r (heads 0..7 hi, then lo), d = 16c .. 16c + 15
       const int st = (warp - 2) * 32 + lane;
@@ -510,8 +518,8 @@ int launch_decode_e4m3_tc(const AttnParams& p_in, const void* pool, void* stream
     OGB_CUDA_CHECK(cudaFuncSetAttribute(paged_decode_e4m3_tc_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     attr_set = true;
   }
-  paged_decode_e4m3_tc_kernel<<<dim3(p.num_seqs * p.num_splits, p.hkv), kTcThreads, kTcSmem, static_cast<cudaStream_t>(stream)>>>(map, p);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_overlapped(paged_decode_e4m3_tc_kernel, dim3(p.num_seqs * p.num_splits, p.hkv), dim3(kTcThreads), kTcSmem,
+                                            static_cast<cudaStream_t>(stream), map, p));
 }
 
 }  // namespace ogb

@@ -226,6 +226,8 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();
   if (dbg && threadIdx.x == 0) dbg[2] = global_timer_ns() - dbg[0];
 
   if (warp < 2) {
@@ -596,8 +598,8 @@ static int launch_prefill_tc(const AttnParams& p, const void* pool, int q_rows, 
     attr_set = true;
   }
   dim3 grid(p.num_tiles, p.hq);
-  paged_prefill_tc_kernel<DK, DV, BN, CHUNKED><<<grid, kFaThreads, Cfg::kSmemBytes, stream>>>(q_map, q16_map, kv_map, p);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_overlapped(paged_prefill_tc_kernel<DK, DV, BN, CHUNKED>, grid, dim3(kFaThreads), Cfg::kSmemBytes, stream, q_map, q16_map,
+                                            kv_map, p));
 }
 
 static unsigned long long* g_fa_dbg = nullptr;

@@ -208,6 +208,22 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n) {
 // on the leader's flags cannot starve it.
 OGB_DEVICE void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// A kernel launched that way (launch_overlapped) may do what depends on no earlier kernel of its stream -- barriers, tensor memory,
+// weights, keys of earlier steps -- and then waits here, in every thread that reads or writes anything else, until the kernels before it
+// have completed and their writes are visible.  A no-op in an ordinary launch.  A kernel that lets its follower start early
+// (pdl_trigger) waits itself before it ends, so that the wait reaches all the way back -- and lets it start only when it holds its own tensor
+// memory: a follower that took the columns first and then waited for this kernel would never end.
+OGB_DEVICE void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A pointer to what earlier kernels wrote, taken anew after the wait.  A __restrict__ pointer lets the compiler move loads ahead of the wait
+// and make them through the read-only path, which need not see those writes; this one has no such promise.
+template <typename T>
+OGB_DEVICE T* after_wait(T* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
+// True inside a model step whose kernels all wait so (ogb_launch_scope of the calling thread).
+bool launch_overlap();
+
 // Process-wide switch for those launches (OGB_TP_PDL=1 or ogb_tp_set_pdl(1); off by default).
 int tp_pdl_enabled();
 
@@ -225,6 +241,11 @@ inline cudaError_t launch_kernel_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 b
   cfg.attrs = pdl ? attr : nullptr;
   cfg.numAttrs = pdl ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return launch_kernel_pdl(kernel, grid, block, smem, stream, launch_overlap(), args...);
 }
 
 // ----------------------------------------------------------------------------------------

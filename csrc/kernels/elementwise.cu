@@ -18,6 +18,10 @@ namespace ogb {
 // ------------------------------------------------------------------------------------------
 __global__ void embedding_kernel(const int* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
                                  __nv_bfloat16* __restrict__ out, int hidden, int vocab, int* status) {
+  // the first kernel of a step: the ones after it start only when everything before the step has completed
+  pdl_wait();
+  pdl_trigger();
+  table = after_wait(table);               // as a gather of rows it reads what the layers left
   const int t = blockIdx.x;
   int id = ids[t];
   if (id < 0 || id >= vocab) {
@@ -26,7 +30,7 @@ __global__ void embedding_kernel(const int* __restrict__ ids, const __nv_bfloat1
   }
   const uint4* src = reinterpret_cast<const uint4*>(table + static_cast<size_t>(id) * hidden);
   uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(t) * hidden);
-  for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) dst[i] = __ldg(src + i);
+  for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) dst[i] = src[i];
 }
 
 // ------------------------------------------------------------------------------------------
@@ -39,6 +43,10 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(__nv_bfloat16* x,
                                                                 const __nv_bfloat16* __restrict__ weight,
                                                                 __nv_bfloat16* __restrict__ out, int hidden, int ldx,
                                                                 int ldo, float eps) {
+  pdl_trigger();
+  pdl_wait();
+  x = after_wait(x);
+  delta = after_wait(delta);
   const int row = blockIdx.x;
   __nv_bfloat16* xr = x + static_cast<size_t>(row) * ldx;
   const __nv_bfloat16* dr = delta ? delta + static_cast<size_t>(row) * hidden : nullptr;
@@ -114,6 +122,10 @@ __global__ void __launch_bounds__(128) rmsnorm_warp_kernel(__nv_bfloat16* x, con
                                                             const __nv_bfloat16* __restrict__ weight,
                                                             __nv_bfloat16* __restrict__ out, int rows, int hidden, int ldx,
                                                             int ldo, float eps) {
+  pdl_trigger();
+  pdl_wait();
+  x = after_wait(x);
+  delta = after_wait(delta);
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -179,6 +191,9 @@ __global__ void __launch_bounds__(128) rmsnorm_warp_kernel(__nv_bfloat16* x, con
 // ------------------------------------------------------------------------------------------
 __global__ void silu_mul_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, int inter,
                                 size_t total_vec) {
+  pdl_trigger();
+  pdl_wait();
+  gu = after_wait(gu);
   const int vec_per_row = inter / 8;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total_vec;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -206,6 +221,9 @@ __global__ void rope_kv_append_kernel(__nv_bfloat16* __restrict__ qkv, const int
                                       void* __restrict__ pool, int hq, int hkv, int d,
                                       int rotary_dim, int interleaved, int page_size, int64_t num_slots, int max_pos,
                                       int* status) {
+  pdl_trigger();
+  pdl_wait();
+  qkv = after_wait(qkv);
   const int t = blockIdx.x;
   int pos = positions[t];
   const int64_t slot = slots[t];  // slot = page * page_size + offset; negative = do not cache
@@ -252,6 +270,9 @@ __global__ void rope_kv_append_kernel(__nv_bfloat16* __restrict__ qkv, const int
 __global__ void rope_kv_append_vec_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions, const int* __restrict__ slots,
                                           const float* __restrict__ cos_sin, __nv_bfloat16* __restrict__ pool, int hq, int hkv, int d, int rotary_dim,
                                           int page_size, int64_t num_slots, int max_pos, int* status) {
+  pdl_trigger();
+  pdl_wait();
+  qkv = after_wait(qkv);
   const int t = blockIdx.x;
   int pos = positions[t];
   const int64_t slot = slots[t];  // slot = page * page_size + offset; negative = do not cache
@@ -313,6 +334,10 @@ __global__ void rope_kv_append_vec_kernel(__nv_bfloat16* __restrict__ qkv, const
 __global__ void kv_append_fp8_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ slots,
                                      uint8_t* __restrict__ pool, float* __restrict__ scales, int hq, int hkv, int d,
                                      int page_size, int64_t num_slots, int fmt, int* status) {
+  pdl_trigger();
+  pdl_wait();
+  qkv = after_wait(qkv);
+  scales = after_wait(scales);
   const float qmax = fmt == 0 ? 448.f : (fmt == 1 ? 127.f : 57344.f);     // fmt 0: e4m3, 1: int8 (symmetric), 2: e5m2
   const int t = blockIdx.x;
   const int64_t slot = slots[t];
@@ -417,9 +442,8 @@ extern "C" int ogb_embedding_bf16(const int* ids, const void* table, void* out, 
                                   int* status, void* stream) {
   if (tokens <= 0) return 0;
   if (hidden % 8) return -3;
-  embedding_kernel<<<tokens, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-      ids, static_cast<const __nv_bfloat16*>(table), static_cast<__nv_bfloat16*>(out), hidden, vocab, status);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_overlapped(embedding_kernel, dim3(tokens), dim3(128), 0, static_cast<cudaStream_t>(stream), ids,
+                                            static_cast<const __nv_bfloat16*>(table), static_cast<__nv_bfloat16*>(out), hidden, vocab, status));
 }
 
 extern "C" int ogb_rmsnorm_bf16(void* x, const void* delta, const void* weight, void* out, int rows, int hidden, int ldx,
@@ -427,15 +451,13 @@ extern "C" int ogb_rmsnorm_bf16(void* x, const void* delta, const void* weight, 
   if (rows <= 0) return 0;
   if (hidden % 8 || ldx % 8 || ldo % 8) return -3;
   if (hidden / 8 <= 32 * kNormWarpMaxVec) {
-    rmsnorm_warp_kernel<<<(rows + 3) / 4, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<__nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(delta), static_cast<const __nv_bfloat16*>(weight),
-        static_cast<__nv_bfloat16*>(out), rows, hidden, ldx, ldo, eps);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(launch_overlapped(rmsnorm_warp_kernel, dim3((rows + 3) / 4), dim3(128), 0, static_cast<cudaStream_t>(stream),
+                                              static_cast<__nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(delta),
+                                              static_cast<const __nv_bfloat16*>(weight), static_cast<__nv_bfloat16*>(out), rows, hidden, ldx, ldo, eps));
   }
-  rmsnorm_kernel<<<rows, kNormThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(delta), static_cast<const __nv_bfloat16*>(weight),
-      static_cast<__nv_bfloat16*>(out), hidden, ldx, ldo, eps);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_overlapped(rmsnorm_kernel, dim3(rows), dim3(kNormThreads), 0, static_cast<cudaStream_t>(stream),
+                                            static_cast<__nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(delta),
+                                            static_cast<const __nv_bfloat16*>(weight), static_cast<__nv_bfloat16*>(out), hidden, ldx, ldo, eps));
 }
 
 extern "C" int ogb_silu_mul_bf16(const void* gate_up, void* out, int rows, int inter, void* stream) {
@@ -445,9 +467,8 @@ extern "C" int ogb_silu_mul_bf16(const void* gate_up, void* out, int rows, int i
   int blocks = static_cast<int>((total_vec + 255) / 256);
   const int cap = ogb_num_sms() * 8;
   if (blocks > cap) blocks = cap;
-  silu_mul_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(gate_up),
-                                                                          static_cast<__nv_bfloat16*>(out), inter, total_vec);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_overlapped(silu_mul_kernel, dim3(blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                                            static_cast<const __nv_bfloat16*>(gate_up), static_cast<__nv_bfloat16*>(out), inter, total_vec));
 }
 
 // Rotation, and the append when pool is not null.
@@ -457,14 +478,12 @@ static cudaError_t launch_rope(void* qkv, const int* positions, const int* slots
                    ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(cos_sin) | reinterpret_cast<uintptr_t>(pool)) & 15) == 0;
   if (vec) {
     const int units = (hq + hkv) * (rotary_dim / 16) + hkv * (d / 8);
-    rope_kv_append_vec_kernel<<<tokens, units < 512 ? (units + 31) / 32 * 32 : 512, 0, stream>>>(
-        static_cast<__nv_bfloat16*>(qkv), positions, slots, cos_sin, static_cast<__nv_bfloat16*>(pool), hq, hkv, d, rotary_dim, page_size, num_slots,
-        max_pos, status);
-  } else {
-    rope_kv_append_kernel<<<tokens, 256, 0, stream>>>(static_cast<__nv_bfloat16*>(qkv), positions, slots, cos_sin, pool, hq, hkv, d, rotary_dim,
-                                                      interleaved, page_size, num_slots, max_pos, status);
+    return launch_overlapped(rope_kv_append_vec_kernel, dim3(tokens), dim3(units < 512 ? (units + 31) / 32 * 32 : 512), 0, stream,
+                             static_cast<__nv_bfloat16*>(qkv), positions, slots, cos_sin, static_cast<__nv_bfloat16*>(pool), hq, hkv, d, rotary_dim,
+                             page_size, num_slots, max_pos, status);
   }
-  return cudaGetLastError();
+  return launch_overlapped(rope_kv_append_kernel, dim3(tokens), dim3(256), 0, stream, static_cast<__nv_bfloat16*>(qkv), positions, slots, cos_sin, pool,
+                           hq, hkv, d, rotary_dim, interleaved, page_size, num_slots, max_pos, status);
 }
 
 extern "C" int ogb_rope_kv_append_bf16(void* qkv, const int* positions, const int* slots, const float* cos_sin,
@@ -483,9 +502,8 @@ static int launch_rope_kv_append_q8(void* qkv, const int* positions, const int* 
   if (d % 8 || rotary_dim % 2 || rotary_dim > d || kv_format < 0 || kv_format > 2) return -3;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   OGB_CUDA_CHECK(launch_rope(qkv, positions, slots, cos_sin, nullptr, tokens, hq, hkv, d, rotary_dim, interleaved, page_size, num_slots, max_pos, status, st));
-  kv_append_fp8_kernel<<<tokens, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(qkv), slots, static_cast<uint8_t*>(pool), scales,
-                                               hq, hkv, d, page_size, num_slots, kv_format, status);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_overlapped(kv_append_fp8_kernel, dim3(tokens), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(qkv), slots,
+                                            static_cast<uint8_t*>(pool), scales, hq, hkv, d, page_size, num_slots, kv_format, status));
 }
 extern "C" int ogb_rope_kv_append_fp8(void* qkv, const int* positions, const int* slots, const float* cos_sin,
                                       void* pool, float* scales, int tokens, int hq, int hkv, int d, int rotary_dim,

@@ -96,12 +96,19 @@ static int rows_launch(Kernel kernel, int grid, int threads, int smem, int split
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = splits;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
-  cfg.numAttrs = splits > 1 ? 1 : 0;
+  if (splits > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = splits;
+    attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  if (launch_overlap()) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
@@ -207,6 +214,7 @@ OGB_DEVICE void rows_epilogue(const RowsGemmParams& p, const ActArgs& act, uint3
   const long long total = static_cast<long long>(p.n_tiles) * k_blocks;
   const int slot_floats = TW * 4 * acc_cols * 32;
   const int rows = p.M;
+  pdl_wait();
   bool ok = true;
   RowsSegs segs(p);
   int tile, kb0, kb1;
@@ -368,6 +376,7 @@ OGB_DEVICE void rows_finish_cluster(const RowsGemmParams& p, const ActArgs& act,
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* stage = reinterpret_cast<float*>(smem);
   bool ok = true;
+  pdl_wait();
   if (warp >= 2 && warp < 6) {
     ok = __all_sync(0xffffffffu, mbar_wait(&tmem_full[0], 0));      // every product has retired: the ring is free
     if (!ok && lane == 0) { atomicOr(p.status, kStatusWaitTimeout); *abort_flag = 1; }
@@ -474,7 +483,7 @@ OGB_DEVICE void rows_tmem(const RowsGemmParams& p, int& acc_cols, int& bufs, uin
 }
 
 template <int TW, int EPI>
-__global__ void __launch_bounds__(kRowsThreads, 2)
+__global__ void __launch_bounds__(kRowsThreads, 1)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a, const RowsGemmParams p, const ActArgs act) {
   extern __shared__ __align__(1024) uint8_t smem[];
   constexpr int kStageW = TW * 128 * kBK * 2;
@@ -491,6 +500,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     tma_prefetch_desc(&tmap_a);
   }
   const uint32_t tmem_base = rows_setup(bars, p.stages, 1, tmem_cols);
+  pdl_trigger();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -498,18 +508,25 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      RowsSegs segs(p);
-      int tile, kb0, kb1;
-      while (ok && segs.next(tile, kb0, kb1)) {
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&bars->empty[stage], phase ^ 1)) { ok = false; break; }
-          uint8_t* sw = smem + stage * stage_bytes;
-          mbar_expect_tx(&bars->full[stage], stage_bytes);
+      auto load_w = [&](const RowsCursor& c, int st) {
+        mbar_expect_tx(&bars->full[st], stage_bytes);
 #pragma unroll
-          for (int w = 0; w < TW; ++w) tma_load_2d(sw + w * 128 * kBK * 2, &tmap_w, &bars->full[stage], kb * kBK, (tile * TW + w) * 128);
-          tma_load_2d(sw + kStageW, &tmap_a, &bars->full[stage], kb * kBK, 0);
-          if (++stage == p.stages) { stage = 0; phase ^= 1; }
+        for (int w = 0; w < TW; ++w)
+          tma_load_2d(smem + st * stage_bytes + w * 128 * kBK * 2, &tmap_w, &bars->full[st], c.kb * kBK, (c.tile * TW + w) * 128);
+      };
+      // the first ring of W is on its way before the kernel ahead has ended; its activations follow
+      int ahead = 0;
+      for (RowsCursor c(p); c.more && ahead < p.stages; c.step()) load_w(c, ahead++);
+      pdl_wait();
+      for (RowsCursor c(p); c.more; c.step()) {
+        if (ahead > 0) {
+          --ahead;
+        } else {
+          if (!mbar_wait(&bars->empty[stage], phase ^ 1)) { ok = false; break; }
+          load_w(c, stage);
         }
+        tma_load_2d(smem + stage * stage_bytes + kStageW, &tmap_a, &bars->full[stage], c.kb * kBK, 0);
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
       if (!ok) { atomicOr(p.status, kStatusWaitTimeout); bars->abort_flag = 1; }
     }

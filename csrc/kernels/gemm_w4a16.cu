@@ -126,6 +126,8 @@ gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
+  if (warp < 6) pdl_wait();
 
   if (warp == 0) {
     // ------------------------------ TMA producer (A) ------------------------------
@@ -431,12 +433,14 @@ gemm_w4_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const RowsGemmPa
   }
   if (threadIdx.x == 0) tma_prefetch_desc(&tmap_a);
   const uint32_t tmem_base = rows_setup(bars, p.stages, 1 + kWDequantWarps, tmem_cols);
+  pdl_trigger();
 
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
+      pdl_wait();                          // the weights are under way meanwhile
       for (RowsCursor c(p); c.more; c.step()) {
         if (!mbar_wait(&bars->empty[stage], phase ^ 1)) { ok = false; break; }
         mbar_expect_tx(&bars->full[stage], static_cast<uint32_t>(p.mn * kWBK * 2));
@@ -577,10 +581,9 @@ static int launch_w4a16_gemm(const void* x, const void* qweight, const void* sca
   }
   const int tiles = ((M + MT * kWTile - 1) / (MT * kWTile)) * ((N + TN - 1) / TN);
   const int grid = tiles < ogb_num_sms() ? tiles : ogb_num_sms();
-  gemm_w4a16_tcgen05_kernel<MT, SF32, TN><<<grid, kWThreads, Cfg::kSmemBytes, stream>>>(
-      ta, static_cast<const uint8_t*>(qweight), scales, static_cast<const uint8_t*>(zp), static_cast<const __nv_bfloat16*>(bias),
-      static_cast<__nv_bfloat16*>(out), M, N, K, ldc, status);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_overlapped(gemm_w4a16_tcgen05_kernel<MT, SF32, TN>, dim3(grid), dim3(kWThreads), Cfg::kSmemBytes, stream, ta,
+                                            static_cast<const uint8_t*>(qweight), scales, static_cast<const uint8_t*>(zp),
+                                            static_cast<const __nv_bfloat16*>(bias), static_cast<__nv_bfloat16*>(out), M, N, K, ldc, status));
 }
 
 }  // namespace ogb

@@ -28,6 +28,9 @@ __global__ void __launch_bounds__(256) moe_route_topk_kernel(const T* __restrict
                                                              float* __restrict__ topk_w,
                                                              int tokens, int experts, int k, int renormalize, int ld, int groups, int keep, bool sigmoid,
                                                              int group_best) {
+  pdl_trigger();
+  pdl_wait();
+  logits = after_wait(logits);
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   __shared__ float s_group[8][kMaxExperts];
   if (warp >= tokens) return;
@@ -195,6 +198,9 @@ __global__ void __launch_bounds__(1024) moe_permute_one_kernel(const int* __rest
                                                                int* __restrict__ route_pos, int* __restrict__ tile_tab, int* __restrict__ meta, int routes,
                                                                int e0, int experts, int max_mtiles) {
   __shared__ int s_cnt[kMaxExperts], s_cur[kMaxExperts];
+  pdl_trigger();
+  pdl_wait();
+  topk_ids = after_wait(topk_ids);
   for (int e = threadIdx.x; e < kMaxExperts; e += blockDim.x) s_cnt[e] = 0;
   __syncthreads();
   for (int i = threadIdx.x; i < routes; i += blockDim.x) {
@@ -249,6 +255,11 @@ __global__ void __launch_bounds__(1024) moe_permute_one_kernel(const int* __rest
 
 __global__ void moe_gather_rows_kernel(const uint4* __restrict__ x, const int* __restrict__ sorted_route, const int* __restrict__ meta,
                                        uint4* __restrict__ xs, int k, int vecs) {
+  pdl_trigger();
+  pdl_wait();
+  x = after_wait(x);
+  sorted_route = after_wait(sorted_route);
+  meta = after_wait(meta);
   const int pos = blockIdx.x;
   if (pos >= meta[1]) return;
   const int token = sorted_route[pos] / k;
@@ -262,6 +273,12 @@ __global__ void moe_gather_rows_kernel(const uint4* __restrict__ x, const int* _
 __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ ys, const int* __restrict__ route_pos,
                                    const float* __restrict__ topk_w, __nv_bfloat16* __restrict__ out, int k, int hidden,
                                    int accumulate) {
+  pdl_trigger();
+  pdl_wait();
+  ys = after_wait(ys);
+  route_pos = after_wait(route_pos);
+  topk_w = after_wait(topk_w);
+  out = after_wait(out);
   const int t = blockIdx.x;
   const int i = blockIdx.y * blockDim.x + threadIdx.x;
   if (i >= hidden / 8) return;
@@ -307,10 +324,8 @@ static int route_topk(const T* logits, const float* bias, int* topk_ids, float* 
   if (groups < 1 || experts % groups != 0 || keep < 1 || keep > groups || k > keep * (experts / groups)) return -3;
   const int warps_per_block = 8;
   const int blocks = (tokens + warps_per_block - 1) / warps_per_block;
-  moe_route_topk_kernel<T><<<blocks, warps_per_block * 32, 0, static_cast<cudaStream_t>(stream)>>>(logits, bias, topk_ids, topk_w, tokens,
-                                                                                                 experts, k, renormalize, ld, groups, keep, sigmoid,
-                                                                                                 group_best);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_overlapped(moe_route_topk_kernel<T>, dim3(blocks), dim3(warps_per_block * 32), 0, static_cast<cudaStream_t>(stream),
+                                            logits, bias, topk_ids, topk_w, tokens, experts, k, renormalize, ld, groups, keep, sigmoid, group_best));
 }
 
 extern "C" int ogb_moe_route_topk(const void* router_logits, int* topk_ids, float* topk_w, int tokens, int experts, int k,
@@ -334,9 +349,8 @@ extern "C" int ogb_moe_permute(const int* topk_ids, int* counts, int* offsets, i
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int routes = tokens * k;
   if (routes <= kPermuteOneRoutes && (reinterpret_cast<uintptr_t>(tile_tab) & 15) == 0) {
-    moe_permute_one_kernel<<<1, routes <= 256 ? 256 : 1024, 0, st>>>(topk_ids, offsets, sorted_route, route_pos, tile_tab, meta, routes, e0, experts,
-                                                                     max_mtiles);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(launch_overlapped(moe_permute_one_kernel, dim3(1), dim3(routes <= 256 ? 256 : 1024), 0, st, topk_ids, offsets, sorted_route,
+                                              route_pos, tile_tab, meta, routes, e0, experts, max_mtiles));
   }
   OGB_CUDA_CHECK(cudaMemsetAsync(counts, 0, sizeof(int) * experts, st));
   moe_count_kernel<<<(routes + 255) / 256, 256, 0, st>>>(topk_ids, counts, routes, e0, experts);
@@ -349,9 +363,9 @@ static int gather_rows(const void* x, const int* sorted_route, const int* meta, 
   if (max_routes <= 0) return 0;
   if (row_bytes % 16) return -3;
   const int vecs = row_bytes / 16;
-  moe_gather_rows_kernel<<<max_routes, vecs < 128 ? (vecs + 31) / 32 * 32 : 128, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint4*>(x), sorted_route, meta, static_cast<uint4*>(xs), k, vecs);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_overlapped(moe_gather_rows_kernel, dim3(max_routes), dim3(vecs < 128 ? (vecs + 31) / 32 * 32 : 128), 0,
+                                            static_cast<cudaStream_t>(stream), static_cast<const uint4*>(x), sorted_route, meta,
+                                            static_cast<uint4*>(xs), k, vecs));
 }
 
 extern "C" int ogb_moe_gather_rows(const void* x, const int* sorted_route, const int* meta, void* xs, int max_routes, int k,
@@ -368,7 +382,7 @@ extern "C" int ogb_moe_combine(const void* ys, const int* route_pos, const float
                                int hidden, int accumulate, void* stream) {
   if (tokens <= 0) return 0;
   if (hidden % 8) return -3;
-  moe_combine_kernel<<<dim3(tokens, (hidden / 8 + 127) / 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(ys), route_pos, topk_w, static_cast<__nv_bfloat16*>(out), k, hidden, accumulate);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_overlapped(moe_combine_kernel, dim3(tokens, (hidden / 8 + 127) / 128), dim3(128), 0, static_cast<cudaStream_t>(stream),
+                                            static_cast<const __nv_bfloat16*>(ys), route_pos, topk_w, static_cast<__nv_bfloat16*>(out), k, hidden,
+                                            accumulate));
 }

@@ -18,8 +18,10 @@ int ogb_gemm_bf16(const void* A, const void* W, void* C, const void* bias, const
                   int N, int K, int lda, int ldw, int ldc, int ldr, int epilogue, int bn, int* status, void* stream);
 
 // Workspace that products with few rows use when the calling thread launches them from now on (null: one per stream): zeroed once,
-// ogb_rows_workspace_bytes(rows) bytes for products of up to `rows` rows, used on one stream at a time.
-void ogb_launch_scope(void* ws, int64_t bytes);
+// ogb_rows_workspace_bytes(rows) bytes for products of up to `rows` rows, used on one stream at a time.  overlap != 0: kernels may start
+// before the one ahead of them has ended, which wants every weight and every key of earlier steps complete when the step's first
+// kernel (the embedding) runs, and decode rows whose newest key alone is of this step.
+void ogb_launch_scope(void* ws, int64_t bytes, int overlap);
 int64_t ogb_rows_workspace_bytes(int rows);
 // ogb_gemm_bf16 whose A rows are delivered by other GPUs: `a_ready` holds one counter per 128-row tile of A, bumped
 // once per 8 rows that land; the TMA producer waits (at most a_wait_ns nanoseconds, 0 = default) for a tile before

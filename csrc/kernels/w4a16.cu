@@ -269,6 +269,8 @@ __global__ void __launch_bounds__(kFusedWarps * 32) w4a16_gemv_fused_kernel(cons
   const int first_tile = blockIdx.x;
   const bool have_w0 = first_tile < num_tiles && (tile_n0(first_tile) < N) && (j0 < min(kb, chunk / 32));
   if (have_w0) w0.load(p, tile_n0(first_tile), j0, kb, zp_stride);
+  pdl_trigger();
+  pdl_wait();
 
   if constexpr (PRO == kProRmsNorm) {
     float ss[MT];
@@ -477,8 +479,7 @@ static int launch_gemv_fused_one(const GemvFusedParams& p, cudaStream_t st) {
     ctas_per_sm = 1;
   // persistent only when the activations stay staged (one chunk); otherwise one tile per CTA as before
   const int blocks = (p.K <= chunk) ? std::min(tiles, ogb_num_sms() * ctas_per_sm) : tiles;
-  kern<<<blocks, kFusedWarps * 32, smem, st>>>(p, chunk, tiles);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_overlapped(kern, dim3(blocks), dim3(kFusedWarps * 32), smem, st, p, chunk, tiles));
 }
 
 template <int MT, int PRO>

@@ -338,6 +338,7 @@ class DecoderModel:
             self.act_q = z(max_tokens, inter_q)
         # fp32 partials of the products with few rows: one buffer, as the products of a step follow one another
         self.gemm_ws = ops.rows_workspace(max(max_tokens, max_seqs), dev) if dev.type == "cuda" else None
+        self.overlap = tp == 1      # a step's kernels start early (ops.launch_scope); peers' rows arrive by protocols of their own
         self.h_last = z(max_seqs, hid)
         self.x_last = z(max_seqs, hid)
         self.logits = z(max_seqs, cfg.vocab)
@@ -489,6 +490,7 @@ class DecoderModel:
             raise ValueError("pipeline stages are built for tp = 1 (one GPU per stage)")
         lo, hi = ranges[stage]
         self.pipeline = (stage, stages)
+        self.overlap = False                             # a later stage does not begin with the embedding
         self.layer_range = (lo, hi)
         if self.native:
             self._native_lib.ogb_decoder_destroy(self.native)
@@ -513,7 +515,9 @@ class DecoderModel:
         """Runs one step; returns logits [num_logit_rows, vocab] (a view of a static buffer)."""
         if self.gemm_ws is None:
             return self._forward(si, kv)
-        with ops.launch_scope(self.gemm_ws):
+        # rows of a verification share new keys, and paged weights arrive during the step: those kernels follow one another
+        overlap = self.overlap and si.verify_table is None and not getattr(self, "weight_packs", None)
+        with ops.launch_scope(self.gemm_ws, overlap):
             return self._forward(si, kv)
 
     def _forward(self, si: StepInputs, kv: KVCache) -> torch.Tensor:

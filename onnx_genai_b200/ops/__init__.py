@@ -255,14 +255,16 @@ def rows_workspace(rows: int, device) -> torch.Tensor:
 
 
 @contextlib.contextmanager
-def launch_scope(workspace: torch.Tensor):
-    """The products that this thread launches inside use ``workspace`` (a model's own: one stream at a time)."""
+def launch_scope(workspace: torch.Tensor, overlap: bool = False):
+    """The products that this thread launches inside use ``workspace`` (a model's own: one stream at a time).  ``overlap``: a kernel may
+    start, and fetch weights and keys of earlier steps, before the one ahead of it has ended; for a step that begins with
+    :func:`embedding` and whose decode rows have one new key each."""
     lib = _native.load()
-    lib.ogb_launch_scope(workspace.data_ptr(), workspace.numel())
+    lib.ogb_launch_scope(workspace.data_ptr(), workspace.numel(), int(overlap))
     try:
         yield
     finally:
-        lib.ogb_launch_scope(0, 0)
+        lib.ogb_launch_scope(0, 0, 0)
 
 
 pack_gate_up = reference.pack_gate_up

@@ -24,7 +24,7 @@ _SIGNATURES = {
     "ogb_num_sms": ([], I),
     "ogb_gemm_bf16": ([P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, P, P], I),
     "ogb_gemm_bf16_wait": ([P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, P, P, ctypes.c_uint64, P, P], I),
-    "ogb_launch_scope": ([P, L], None),
+    "ogb_launch_scope": ([P, L, I], None),
     "ogb_rows_workspace_bytes": ([I], L),
     "ogb_gemm_set_stream_k": ([I], I),
     "ogb_tp_set_pdl": ([I], I),
