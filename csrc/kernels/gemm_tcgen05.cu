@@ -946,8 +946,8 @@ static int gemm_bf16_dispatch(const void* A, const void* W, void* C, const void*
   if (epilogue == kEpiSwiGLU && (bn < 64 || (N % bn) != 0 || C_f32 != nullptr)) return -6;
   if (batch.count < 1 || (batch.a_step % 8) != 0 || (batch.c_step % 8) != 0 || (batch.count > 1 && (a_ready != nullptr || epilogue != kEpiNone))) return -9;
   // Few rows: gemm_rows.cuh.  Where the line lies, in us on B200 with weights from HBM, tile kernel -> this one (floor):
-  //   tiles of 128 columns for at most one wave, clusters over K: better at all sizes it takes.  N x K = 4608 x 3584 (5): 26.7 -> 11.2 at 1
-  //     row, 21.5 -> 18.5 at 256; 3584 x 18944 (21): 85.9 -> 29.8, 110 -> 47.1; 128 x 2048: 12.4 -> 5.9, 12.7 -> 10.8
+  //   tiles of 128 columns for at most one wave, clusters over K: better at all sizes it takes.  N x K = 4608 x 3584 (5): 26.7 -> 12.9 at 1
+  //     row, 21.5 -> 18.9 at 256; 3584 x 18944 (21): 85.9 -> 31.4, 110 -> 48.0; 128 x 2048: 12.4 -> 7.1, 12.7 -> 11.7
   //   more tiles, ranges: 152064 x 3584 (169): 225 -> 170 at 1 row, 185 -> 177 at 40, 188 -> 184 at 77, 193 -> 200 at 128; 151936 x 896 (42):
   //     65 -> 53, 66 -> 63, 54 -> 71, 58 -> 84: the epilogue of a tile is as long as its few k-blocks
   //   gated 37888 x 3584 (42): 57 -> 49 at 16, 49.2 -> 50.0 at 40, 49.6 -> 53.2 at 77: one tile per SM, whose epilogue nothing hides
