@@ -14,8 +14,9 @@
 //                online softmax in the log2 domain
 //   prefill      one CTA = 64 query rows of one head; causal (+ optional sliding window)
 //   decode       one CTA = (sequence, kv head, KV split); the G query heads of the group are the
-//                MMA rows, each warp takes one page of every block, warps merge at the end;
-//                splits > 1 write partials that paged_decode_merge_kernel combines
+//                MMA rows, each warp takes one page of every block, warps merge at the end; in small launches
+//                up to 8 splits are a cluster and merge through shared memory, elsewhere they
+//                write partials that paged_decode_merge_kernel combines
 // Page ids are bounds-checked: a bad id raises kStatusIndexOutOfRange and page 0 is read instead.
 #include <mutex>
 #include <unordered_map>
@@ -225,6 +226,9 @@ __global__ void __launch_bounds__(kAttnThreads, 2) paged_decode_kernel(const __g
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(sq + Cfg::kQBytes);
   uint64_t* empty_bar = full_bar + Cfg::kStages;
   float* sm_ml = reinterpret_cast<float*>(empty_bar + Cfg::kStages);  // [4 warps][16 rows][2]
+  float* sm_o = reinterpret_cast<float*>(stages);                     // once the ring is drained: [4][16][D] fp32 ...
+  float* fin_acc = sm_o + 4 * 16 * D;                                 // ... and, for a cluster, this CTA's [G][D]
+  float* fin_ml = sm_ml + 4 * 16 * 2;                                 // and [G][2]
 
   pdl_trigger();
   const int seq = blockIdx.x / p.num_splits;
@@ -246,6 +250,11 @@ __global__ void __launch_bounds__(kAttnThreads, 2) paged_decode_kernel(const __g
   if (b_begin >= b_end) {
     // nothing to do for this split (or an inactive row): publish an empty partial
     pdl_wait();
+    if (p.cluster_merge != 0 && ctx > 0) {
+      if (threadIdx.x < 16) { fin_ml[threadIdx.x * 2] = -INFINITY; fin_ml[threadIdx.x * 2 + 1] = 0.f; }
+      decode_merge_cluster<D>(p, fin_acc, fin_ml, seq, kvh, split);
+      return;
+    }
     if (p.num_splits > 1 && ctx > 0) {
       for (int idx = threadIdx.x; idx < G * D; idx += blockDim.x) {
         const int r = idx / D, d = idx % D;
@@ -269,6 +278,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2) paged_decode_kernel(const __g
       if (!attn_produce<Cfg>(&kv_map, p, stages, full_bar, empty_bar, seq, kvh, ctx, blocks, b_begin, b_end, ctx - 1))
         atomicOr(p.status, kStatusWaitTimeout);
     }
+    __syncwarp();
+    if (p.cluster_merge != 0) decode_merge_cluster<D>(p, fin_acc, fin_ml, seq, kvh, split);
     return;
   }
 
@@ -374,7 +385,6 @@ __global__ void __launch_bounds__(kAttnThreads, 2) paged_decode_kernel(const __g
 
   // ---- merge the four warps (each saw a disjoint quarter of the keys) ----
   compute_bar_sync();  // every stage has been consumed: the ring can be reused as scratch
-  float* sm_o = reinterpret_cast<float*>(stages);  // [4][16][D] fp32
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     float l = l_run[r];
@@ -409,12 +419,16 @@ __global__ void __launch_bounds__(kAttnThreads, 2) paged_decode_kernel(const __g
     const int head = kvh * G + row;
     if (p.num_splits == 1) {
       p.out[static_cast<size_t>(seq) * p.o_stride + head * D + d] = __float2bfloat16(l > 0.f ? acc / l : 0.f);
+    } else if (p.cluster_merge != 0) {
+      fin_acc[idx] = acc;
+      if (d == 0) { fin_ml[row * 2] = mx; fin_ml[row * 2 + 1] = l; }
     } else {
       const size_t slot = (static_cast<size_t>(seq) * p.hq + head) * p.num_splits + split;
       p.part_o[slot * D + d] = acc;
       if (d == 0) { p.part_ml[slot * 2] = mx; p.part_ml[slot * 2 + 1] = l; }
     }
   }
+  if (p.cluster_merge != 0) decode_merge_cluster<D>(p, fin_acc, fin_ml, seq, kvh, split);
 }
 
 __global__ void paged_decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
@@ -504,9 +518,10 @@ static int launch_decode(const CUtensorMap& map, const AttnParams& p, cudaStream
     attr_set = true;
   }
   dim3 grid(p.num_seqs * p.num_splits, p.hkv);
-  int rc = static_cast<int>(launch_overlapped(paged_decode_kernel<D>, grid, dim3(kAttnThreads), Cfg::kSmemBytes, stream, map, p));
+  AttnParams pc = p;
+  int rc = launch_decode_clustered(paged_decode_kernel<D>, grid, Cfg::kSmemBytes, stream, map, pc);
   if (rc != 0) return rc;
-  if (p.num_splits > 1) {
+  if (p.num_splits > 1 && pc.cluster_merge == 0) {
     dim3 mgrid(p.num_seqs, p.hq);
     rc = static_cast<int>(launch_overlapped(paged_decode_merge_kernel, mgrid, dim3(D), 0, stream, p.part_o, p.part_ml, p.ctx_len, p.out, p.hq, D,
                                             p.num_splits, p.o_stride));

@@ -171,6 +171,9 @@ __global__ void __launch_bounds__(kAttnThreads) paged_decode_fp8_kernel(const __
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(sq + 16 * kD * 2);
   uint64_t* empty_bar = full_bar + kDecStages;
   float* sm_ml = reinterpret_cast<float*>(empty_bar + kDecStages);
+  float* sm_o = reinterpret_cast<float*>(stages);         // once the ring is drained: [4][16][128] fp32 = 32 KB of its 48 ...
+  float* fin_acc = sm_o + 4 * 16 * kD;                    // ... and, for a cluster, this CTA's [G][128]
+  float* fin_ml = sm_ml + 4 * 16 * 2;                     // and [G][2]
 
   pdl_trigger();
   const int seq = blockIdx.x / p.num_splits, split = blockIdx.x % p.num_splits, kvh = blockIdx.y;
@@ -189,6 +192,11 @@ __global__ void __launch_bounds__(kAttnThreads) paged_decode_fp8_kernel(const __
   }
   if (b_begin >= b_end) {
     pdl_wait();
+    if (p.cluster_merge != 0 && ctx > 0) {
+      if (threadIdx.x < 16) { fin_ml[threadIdx.x * 2] = -INFINITY; fin_ml[threadIdx.x * 2 + 1] = 0.f; }
+      decode_merge_cluster<kD>(p, fin_acc, fin_ml, seq, kvh, split);
+      return;
+    }
     if (p.num_splits > 1 && ctx > 0) {
       for (int idx = threadIdx.x; idx < G * kD; idx += blockDim.x) {
         const int r = idx / kD, d = idx % kD;
@@ -208,6 +216,8 @@ __global__ void __launch_bounds__(kAttnThreads) paged_decode_fp8_kernel(const __
   if (warp == 4) {
     if (lane == 0 && !fp8_produce(&kv_map, p, stages, full_bar, empty_bar, kDecStages, seq, kvh, ctx, b_begin, b_end, kv_lo, ctx - 1))
       atomicOr(p.status, kStatusWaitTimeout);
+    __syncwarp();
+    if (p.cluster_merge != 0) decode_merge_cluster<kD>(p, fin_acc, fin_ml, seq, kvh, split);
     return;
   }
   pdl_wait();
@@ -321,7 +331,6 @@ __global__ void __launch_bounds__(kAttnThreads) paged_decode_fp8_kernel(const __
   if (!ok && lane == 0) atomicOr(p.status, kStatusWaitTimeout);
 
   compute_bar_sync();
-  float* sm_o = reinterpret_cast<float*>(stages);   // [4][16][128] fp32 = 32 KB <= 48 KB of ring
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     float l = l_run[r];
@@ -353,12 +362,16 @@ __global__ void __launch_bounds__(kAttnThreads) paged_decode_fp8_kernel(const __
     const int head = kvh * G + row;
     if (p.num_splits == 1) {
       p.out[static_cast<size_t>(seq) * p.o_stride + head * kD + d] = __float2bfloat16(l > 0.f ? acc / l : 0.f);
+    } else if (p.cluster_merge != 0) {
+      fin_acc[idx] = acc;
+      if (d == 0) { fin_ml[row * 2] = mx; fin_ml[row * 2 + 1] = l; }
     } else {
       const size_t slot = (static_cast<size_t>(seq) * p.hq + head) * p.num_splits + split;
       p.part_o[slot * kD + d] = acc;
       if (d == 0) { p.part_ml[slot * 2] = mx; p.part_ml[slot * 2 + 1] = l; }
     }
   }
+  if (p.cluster_merge != 0) decode_merge_cluster<kD>(p, fin_acc, fin_ml, seq, kvh, split);
 }
 
 __global__ void paged_decode_fp8_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
@@ -1040,10 +1053,11 @@ static int launch_decode_q(const void* q, void* out, const void* pool, const flo
     }
     OGB_CUDA_CHECK(launch_overlapped(paged_decode_e4m3_mma_kernel, dim3(num_seqs * num_splits, hkv), dim3(kAttnThreads), kMmaSmem, st, map, p));
   } else {
-    OGB_CUDA_CHECK(launch_overlapped(paged_decode_fp8_kernel, dim3(num_seqs * num_splits, hkv), dim3(kAttnThreads), kDecSmem, st, map, p));
+    rc = launch_decode_clustered(paged_decode_fp8_kernel, dim3(num_seqs * num_splits, hkv), kDecSmem, st, map, p);
+    if (rc != 0) return rc;
   }
   rc = static_cast<int>(cudaGetLastError());
-  if (rc == 0 && num_splits > 1) {
+  if (rc == 0 && num_splits > 1 && p.cluster_merge == 0) {
     rc = static_cast<int>(launch_overlapped(paged_decode_fp8_merge_kernel, dim3(num_seqs, hq), dim3(kD), 0, st, part_o, part_ml, ctx_len, p.out, hq,
                                             num_splits, o_stride));
   }
