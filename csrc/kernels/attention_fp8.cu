@@ -1088,7 +1088,7 @@ static int launch_prefill_q(const void* q, void* out, const void* pool, const fl
   // the keys among as many CTAs as two per SM leave room for.  8-byte stores of the merge want an even output stride.
   const int ctas = num_tiles * hkv * ((p.group + 3) / 4);
   int splits = 1;
-  while (splits < 8 && 2 * splits * ctas <= 2 * ogb_num_sms() && (o_stride % 4) == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0) splits *= 2;
+  while (!tile_sums() && splits < 8 && 2 * splits * ctas <= 2 * ogb_num_sms() && (o_stride % 4) == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0) splits *= 2;
   p.num_splits = splits;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(num_tiles * splits, hq);

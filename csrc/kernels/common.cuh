@@ -223,6 +223,8 @@ OGB_DEVICE T* after_wait(T* p) {
 }
 // True inside a model step whose kernels all wait so (ogb_launch_scope of the calling thread).
 bool launch_overlap();
+// True where the order of sums must not depend on kernels for few rows (ogb_tile_sums of the calling thread).
+bool tile_sums();
 
 // Process-wide switch for those launches (OGB_TP_PDL=1 or ogb_tp_set_pdl(1); off by default).
 int tp_pdl_enabled();

@@ -47,7 +47,7 @@ OGB_DEVICE float plain_act(const ActArgs& act, float v) {
 // With more tiles than CTAs only those of about the last wave are cut (sk_cut_tiles), and they come first: the whole waves that follow
 // are dealt round-robin, so that CTAs walk K in step and share what they read through L2 (cut from end to end, 7100 rows
 // against a 3584 x 18944 projection drew every operand from HBM again and again: 1101 us), and a fix-up's wait passes
-// under the main loop of the tile after it.
+// under the main loop of the tile after it.  Where the order of the sums must stay (tile_sums), all tiles are cut.
 // ----------------------------------------------------------------------------------------
 // Tiles of many rows: 16 tiles of A at a time against every tile of W, so that the tiles under way at one moment (about 148) span
 // 2048 rows of A and 2400 of W instead of all of A and two tiles of W.
@@ -69,7 +69,7 @@ OGB_DEVICE void raster_tile(int tile, int m_tiles, int n_tiles, bool grouped, in
 
 // How many of a launch's first tiles stream-K cuts into ranges: all when there are fewer than CTAs, else those of the incomplete last wave,
 // and a wave more where they are so few that many CTAs would share each of them.
-__host__ __device__ inline int sk_cut_tiles(int tiles, int ctas) {
+inline int sk_cut_tiles(int tiles, int ctas) {
   if (tiles <= ctas) return tiles;
   const int rest = tiles % ctas;
   return 2 * ctas > 7 * rest ? rest + ctas : rest;
@@ -93,9 +93,9 @@ struct GemmWork {
     const long long cut = (base + 1) * rem;
     return i < cut ? static_cast<int>(i / (base + 1)) : static_cast<int>(rem + (i - cut) / base);
   }
-  OGB_DEVICE GemmWork(bool stream_k, int tiles, int kblocks) : k_blocks(kblocks), num_tiles(tiles) {
+  // cut: how many of the first tiles are cut into ranges (0: no stream-K)
+  OGB_DEVICE GemmWork(int cut, int tiles, int kblocks) : k_blocks(kblocks), num_tiles(tiles) {
     stride = gridDim.x;
-    const int cut = stream_k ? sk_cut_tiles(tiles, stride) : 0;
     tile = cut + blockIdx.x;
     sk_total = static_cast<long long>(cut) * kblocks;
     it = range_begin(sk_total, stride, blockIdx.x);

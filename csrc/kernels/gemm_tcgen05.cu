@@ -68,6 +68,7 @@ struct GemmCfg {
 struct GemmBatch {
   int count = 1, a_step = 0, c_step = 0, page_d = 0;
   int raster = 0;      // tiles in groups of kRasterM tiles of A (raster_tile)
+  int cut = 0;         // stream-K: how many of the first tiles are cut into ranges
 };
 
 // fp32 partial accumulators of stream-K: slot = CTA, layout [BN / 32 column chunks][128 rows][32 floats], so a warp's
@@ -162,7 +163,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       uint32_t phase = 0;
       bool ok = true;
       unsigned long long seen_ready = 0ull;     // m-tiles (of the first 64) whose rows are known to have arrived
-      GemmWork work(stream_k, num_tiles, k_blocks);
+      GemmWork work(batch.cut, num_tiles, k_blocks);
       GemmSeg seg;
       while (ok && work.next(seg)) {
         const int z = seg.tile / batch_tiles;
@@ -210,7 +211,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       uint32_t phase = 0;
       bool ok = true;
       int it = 0;
-      GemmWork work(stream_k, num_tiles, k_blocks);
+      GemmWork work(batch.cut, num_tiles, k_blocks);
       GemmSeg seg;
       for (; ok && work.next(seg); ++it) {
         const int acc = it & 1;
@@ -242,7 +243,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     bool ok = true;
     int it = 0;
-    GemmWork work(stream_k, num_tiles, k_blocks);
+    GemmWork work(batch.cut, num_tiles, k_blocks);
     GemmSeg seg;
     const long long sk_total = work.sk_total;
     for (; ok && work.next(seg); ++it) {
@@ -495,7 +496,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         const int q = lane;  // row quarter of the tile = TMEM quarter of the epilogue warp that stores it
         uint32_t done = 0;
         bool ok = true;
-        GemmWork work(stream_k, num_tiles, k_blocks);
+        GemmWork work(batch.cut, num_tiles, k_blocks);
         GemmSeg seg;
         while (ok && work.next(seg)) {
           if (seg.kb1 < k_blocks) continue;            // a partial segment stores nothing: its finisher signals the tile
@@ -696,6 +697,10 @@ static SkWorkspace* sk_workspace(cudaStream_t stream, int ctas) {
   return &w;
 }
 
+// Products of this thread take the tile kernel, with all tiles cut where stream-K applies, whatever their rows (ogb_tile_sums).
+static thread_local bool g_tile_sums = false;
+bool tile_sums() { return g_tile_sums; }
+
 static int g_stream_k = -1;     // -1: read OGB_STREAM_K once (default on); 0 / 1 set by ogb_gemm_set_stream_k
 
 static bool stream_k_enabled() {
@@ -720,9 +725,16 @@ constexpr float kSkShared = 6.0f;
 // are long enough.  A CTA's partial costs about 25 k-blocks to write and add (0.3 us each at 256 columns): 7100 and 2304 rows against
 // 3584 x 18944 gain 1244 -> 690 and 298 -> 234 us; with K = 3584 (2304 rows: 54 -> 71 us) the fix-ups are what is left.
 constexpr float kSkPartial = 25.0f;
+// A launch's rule: the fix-up's cost, and whether all tiles are cut.
+struct SkRule {
+  float fix;
+  bool all;
+  int cut(int tiles, int sms) const { return all ? tiles : sk_cut_tiles(tiles, sms); }
+};
 // The cost of the fix-ups of a launch, in k-blocks.
-static float sk_fix(int tiles, int k_blocks, int sms, float fix) {
-  const int cut = sk_cut_tiles(tiles, sms);
+static float sk_fix(int tiles, int k_blocks, int sms, SkRule rule) {
+  const float fix = rule.fix;
+  const int cut = rule.cut(tiles, sms);
   const float shared = static_cast<float>(sms) / static_cast<float>(std::max(cut, 1));
   if (cut < tiles) {
     const float own = kSkPartial * (1.f + shared);
@@ -730,18 +742,18 @@ static float sk_fix(int tiles, int k_blocks, int sms, float fix) {
   }
   return shared > kSkShared ? fix * shared / kSkShared : fix;
 }
-static bool stream_k_applies(int tiles, int k_blocks, int sms, float fix) {
+static bool stream_k_applies(int tiles, int k_blocks, int sms, SkRule rule) {
   if (!stream_k_enabled() || tiles % sms == 0 || static_cast<long long>(tiles) * k_blocks < 2LL * sms) return false;
   const float w = static_cast<float>(tiles) / static_cast<float>(sms);
   const float dp = static_cast<float>((tiles + sms - 1) / sms);
-  const float sk = w + sk_fix(tiles, k_blocks, sms, fix) / static_cast<float>(k_blocks);
+  const float sk = w + sk_fix(tiles, k_blocks, sms, rule) / static_cast<float>(k_blocks);
   return sk < 0.93f * dp;
 }
 // Relative duration of a launch with `tiles` tiles of relative cost `cost`: whole waves when tiles are dealt
 // round-robin, the exact share plus the fix-up when stream-K spreads the k-blocks evenly.
-static float launch_cost(int tiles, int k_blocks, int sms, float cost, float fix) {
-  if (stream_k_applies(tiles, k_blocks, sms, fix))
-    return (static_cast<float>(tiles) / static_cast<float>(sms) + sk_fix(tiles, k_blocks, sms, fix) / static_cast<float>(k_blocks)) * cost;
+static float launch_cost(int tiles, int k_blocks, int sms, float cost, SkRule rule) {
+  if (stream_k_applies(tiles, k_blocks, sms, rule))
+    return (static_cast<float>(tiles) / static_cast<float>(sms) + sk_fix(tiles, k_blocks, sms, rule) / static_cast<float>(k_blocks)) * cost;
   return static_cast<float>((tiles + sms - 1) / sms) * cost;
 }
 
@@ -774,11 +786,13 @@ static int launch_gemm(const void* A, const void* W, void* C, const void* bias, 
   uint32_t* sk_flags = nullptr;
   uint32_t sk_seq = 0;
   const int k_blocks = (K + kBK - 1) / kBK;
-  batch.raster = group_tab == nullptr && batch.count == 1 && static_cast<long long>(M) * K * 2 > kRasterBytes;
-  if (group_tab == nullptr && stream_k_applies(tiles, k_blocks, sms, EPI == kEpiScatter ? kSkFixScatter : kSkFixPlain)) {
+  batch.raster = group_tab == nullptr && batch.count == 1 && !tile_sums() && static_cast<long long>(M) * K * 2 > kRasterBytes;
+  const SkRule rule{EPI == kEpiScatter ? kSkFixScatter : kSkFixPlain, tile_sums()};
+  if (group_tab == nullptr && stream_k_applies(tiles, k_blocks, sms, rule)) {
     SkWorkspace* w = sk_workspace(stream, sms);
     if (w != nullptr) {
       grid = sms;
+      batch.cut = rule.cut(tiles, sms);
       sk_ws = w->ws;
       sk_flags = w->flags;
       sk_seq = ++w->seq;
@@ -896,6 +910,15 @@ using namespace ogb;
 extern "C" void ogb_launch_scope(void* ws, int64_t bytes, int overlap) {
   g_scope = LaunchScope{ws, static_cast<size_t>(ws != nullptr ? bytes : 0), overlap != 0};
 }
+// The order of a product's sums over K then depends on its sizes as the tile kernel alone divides them, and 8-bit prompts are not split
+// over their keys.  For models that choose among experts: a sum in another order moves a row's scores in their last bits, two experts that
+// score alike change places, and one of them is 3 % of the row's logits (24 requests of 1 - 45 sequences of the 30B shape with products of few
+// rows in clusters: 5 differ by 0.030 - 0.044, the others by 0.005 - 0.022).  Returns the thread's old setting.
+extern "C" int ogb_tile_sums(int on) {
+  const int old = g_tile_sums ? 1 : 0;
+  g_tile_sums = on != 0;
+  return old;
+}
 extern "C" int64_t ogb_rows_workspace_bytes(int rows) {
   const int mn = std::min(kRowsRangesM, (std::max(rows, 1) + 15) / 16 * 16);
   const int sms = ogb_num_sms();
@@ -952,7 +975,7 @@ static int gemm_bf16_dispatch(const void* A, const void* W, void* C, const void*
   //     65 -> 53, 66 -> 63, 54 -> 71, 58 -> 84: the epilogue of a tile is as long as its few k-blocks
   //   gated 37888 x 3584 (42): 57 -> 49 at 16, 49.2 -> 50.0 at 40, 49.6 -> 53.2 at 77: one tile per SM, whose epilogue nothing hides
   const int rows_max = epilogue == kEpiSwiGLU ? kRowsGatedM : (N + 127) / 128 > ogb_num_sms() ? kRowsRangesM : kRowsMaxM;
-  if (M <= rows_max && a_ready == nullptr && batch.count == 1 && batch.page_d == 0 && (epilogue == kEpiSwiGLU ? bn == 256 : bn == 0)) {
+  if (M <= rows_max && !tile_sums() && a_ready == nullptr && batch.count == 1 && batch.page_d == 0 && (epilogue == kEpiSwiGLU ? bn == 256 : bn == 0)) {
     const int rc = launch_rows(A, W, C, bias, residual, C_f32, M, N, K, lda, ldw, ldc, ldr, epilogue, act, status, stream);
     if (rc != kRowsDeclined) return rc;
   }
@@ -972,7 +995,7 @@ static int gemm_bf16_dispatch(const void* A, const void* W, void* C, const void*
     for (int i = 0; i < 5; ++i) {
       if (cand[i] < 128 && m_tiles > 3) break;  // narrow tiles only pay off for decode-sized M
       const int tiles = m_tiles * ((N + cand[i] - 1) / cand[i]) * batch.count;
-      const float t = launch_cost(tiles, (K + kBK - 1) / kBK, sms, cost[i], kSkFixPlain);
+      const float t = launch_cost(tiles, (K + kBK - 1) / kBK, sms, cost[i], SkRule{kSkFixPlain, tile_sums()});
       if (t < best - 1e-6f) { best = t; bn = cand[i]; }
     }
   }
@@ -1049,7 +1072,7 @@ extern "C" int ogb_gemm_bf16_scatter(const void* A, const void* W, int M, int N,
     bn = 256;
     for (int i = 0; i < 3; ++i) {
       const int tiles = m_tiles * ((N + cand[i] - 1) / cand[i]);
-      const float t = launch_cost(tiles, (K + kBK - 1) / kBK, sms, cost[i], kSkFixScatter);
+      const float t = launch_cost(tiles, (K + kBK - 1) / kBK, sms, cost[i], SkRule{kSkFixScatter, tile_sums()});
       if (t < best - 1e-6f) { best = t; bn = cand[i]; }
     }
   }

@@ -23,6 +23,9 @@ int ogb_gemm_bf16(const void* A, const void* W, void* C, const void* bias, const
 // kernel (the embedding) runs, and decode rows whose newest key alone is of this step.
 void ogb_launch_scope(void* ws, int64_t bytes, int overlap);
 int64_t ogb_rows_workspace_bytes(int rows);
+// on != 0: products that the calling thread launches from now on sum over K as the tile kernel alone does, whatever their rows (models
+// that choose among experts).  Returns the old setting.
+int ogb_tile_sums(int on);
 // ogb_gemm_bf16 whose A rows are delivered by other GPUs: `a_ready` holds one counter per 128-row tile of A, bumped
 // once per 8 rows that land; the TMA producer waits (at most a_wait_ns nanoseconds, 0 = default) for a tile before
 // loading it, and the last CTA to finish clears the counters (a_done: a zeroed word).

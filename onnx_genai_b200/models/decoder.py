@@ -517,7 +517,7 @@ class DecoderModel:
             return self._forward(si, kv)
         # rows of a verification share new keys, and paged weights arrive during the step: those kernels follow one another
         overlap = self.overlap and si.verify_table is None and not getattr(self, "weight_packs", None)
-        with ops.launch_scope(self.gemm_ws, overlap):
+        with ops.launch_scope(self.gemm_ws, overlap), ops.tile_sums(bool(self.cfg.moe.num_experts)):
             return self._forward(si, kv)
 
     def _forward(self, si: StepInputs, kv: KVCache) -> torch.Tensor:
@@ -637,7 +637,7 @@ class DecoderModel:
         hl = self.h_last[:r]
         self._norm(xl, w.final_norm, None, hl)
         logits = self.logits[:r]
-        self._gemm(hl, w.lm_head, out=logits)
+        self._head(hl, logits)
         return logits
 
     def _attention(self, si, kv, li, qkv, attn):
@@ -697,7 +697,7 @@ class DecoderModel:
         hl = self.h_last[:r]
         torch.index_select(h, 0, si.logit_rows[:r].long(), out=hl)
         logits = self.logits[:r]
-        self._gemm(hl, w.lm_head, out=logits)
+        self._head(hl, logits)
         return logits
 
     # --------------------------------------------------------------------------------------
@@ -712,6 +712,12 @@ class DecoderModel:
             ops.gemm(a, wt, bias=bias, out=out)
         else:
             out.copy_(ops.gemm(a, wt, bias=bias))
+
+    def _head(self, hl, logits):
+        if not hl.is_cuda:
+            return self._gemm(hl, self.w.lm_head, out=logits)
+        with ops.tile_sums(False):                       # no experts are chosen behind it
+            self._gemm(hl, self.w.lm_head, out=logits)
 
     def _row_parallel(self, a, wt, x, slot=0):
         """x += a @ wt^T.  TP=1: fused residual epilogue.  TP>1: partial sum -> all-reduce -> returned as

@@ -25,8 +25,7 @@ def moe_forward(model, h, lw, x):
         ws = moe_ops.MoEWorkspace(model.max_tokens, cfg.moe.top_k, e_local, cfg.hidden, cfg.moe.expert_intermediate,
                                   model.device, h.dtype)
         model._moe_ws = ws
-    # 32 bits on the GPU: rounded to bf16, near-equal scores change places
-    router_logits = ops.gemm(h, lw.router_w, out_f32=h.is_cuda)
+    router_logits = ops.gemm(h, lw.router_w)
     if model.tp == 1:
         moe_ops.moe_experts(h, router_logits, lw.expert_gate_up, lw.expert_down, ws, x, cfg.moe.top_k, cfg.moe.renormalize,
                             model.w.swiglu_half, e0, accumulate=True)

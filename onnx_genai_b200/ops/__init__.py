@@ -267,6 +267,18 @@ def launch_scope(workspace: torch.Tensor, overlap: bool = False):
         lib.ogb_launch_scope(0, 0, 0)
 
 
+@contextlib.contextmanager
+def tile_sums(on: bool = True):
+    """The products that this thread launches inside sum over K as the tile kernel alone does, whatever their rows: for models that choose
+    among experts, where sums in another order make experts of equal score change places."""
+    lib = _native.load()
+    old = lib.ogb_tile_sums(int(on))
+    try:
+        yield
+    finally:
+        lib.ogb_tile_sums(old)
+
+
 pack_gate_up = reference.pack_gate_up
 
 
