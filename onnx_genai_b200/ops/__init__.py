@@ -12,6 +12,7 @@ import collections
 import contextlib
 import math
 import os
+import threading
 
 import torch
 
@@ -254,17 +255,29 @@ def rows_workspace(rows: int, device) -> torch.Tensor:
     return torch.zeros(n, dtype=torch.uint8, device=device)
 
 
+_scopes = threading.local()      # .now: the (workspace, overlap) of the calling thread's innermost scope
+
+
 @contextlib.contextmanager
 def launch_scope(workspace: torch.Tensor, overlap: bool = False):
     """The products that this thread launches inside use ``workspace`` (a model's own: one stream at a time).  ``overlap``: a kernel may
     start, and fetch weights and keys of earlier steps, before the one ahead of it has ended; for a step that begins with
-    :func:`embedding` and whose decode rows have one new key each."""
+    :func:`embedding` and whose decode rows have one new key each.  A scope around this one holds again behind it."""
     lib = _native.load()
-    lib.ogb_launch_scope(workspace.data_ptr(), workspace.numel(), int(overlap))
+
+    def enter(scope):
+        _scopes.now = scope
+        if scope is None:
+            lib.ogb_launch_scope(0, 0, 0)
+        else:
+            lib.ogb_launch_scope(scope[0].data_ptr(), scope[0].numel(), int(scope[1]))
+
+    around = getattr(_scopes, "now", None)
+    enter((workspace, overlap))
     try:
         yield
     finally:
-        lib.ogb_launch_scope(0, 0, 0)
+        enter(around)
 
 
 @contextlib.contextmanager
