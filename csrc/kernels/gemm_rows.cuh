@@ -53,10 +53,10 @@ struct RowsGemmParams {
   unsigned int* counters;                   // ranges: [CTA], zero between launches
 };
 
-// The workspace of a launch of at most `ctas` CTAs: the calling thread's (ogb_launch_scope) or the stream's; null when there is none
-// (a capture outside a step) -- the product is then not one for these kernels (kRowsDeclined).
+// The calling thread's workspace (ogb_launch_scope) where it is large enough for a launch of at most `ctas` CTAs; null: the product is not
+// one for these kernels (kRowsDeclined).
 constexpr int kRowsDeclined = INT32_MIN;
-void* rows_workspace(cudaStream_t stream, int ctas, int tw, int mn);
+void* rows_workspace(int ctas, int tw, int mn);
 size_t rows_counter_bytes(int ctas);
 
 // CTAs per tile: as many as can run at once in clusters (whole clusters have to fit the hardware's groups of SMs, which the driver knows) and

@@ -686,7 +686,7 @@ static SkWorkspace* sk_workspace(cudaStream_t stream, int ctas) {
     const size_t bytes = static_cast<size_t>(ctas) * kBM * 256 * sizeof(float);
     if (cudaMalloc(&w.ws, bytes) != cudaSuccess) { w.ws = nullptr; return nullptr; }
     if (cudaMalloc(&w.flags, static_cast<size_t>(ctas) * 4 * sizeof(uint32_t)) != cudaSuccess ||
-        cudaMemset(w.flags, 0, static_cast<size_t>(ctas) * 4 * sizeof(uint32_t)) != cudaSuccess) {
+        cudaMemsetAsync(w.flags, 0, static_cast<size_t>(ctas) * 4 * sizeof(uint32_t), stream) != cudaSuccess) {
       cudaFree(w.ws);
       w.ws = nullptr;
       return nullptr;
@@ -812,9 +812,9 @@ static int launch_gemm(const void* A, const void* W, void* C, const void* bias, 
 // ----------------------------------------------------------------------------------------
 // products with few rows (gemm_rows.cuh)
 // ----------------------------------------------------------------------------------------
-// Workspace of the products that one thread launches for a model step: the model's own buffer (its steps follow one another, so its
-// products can share it, replayed graphs included), zeroed when it was made.  Without one -- a call outside a step -- the buffer
-// belongs to the stream, and a capture that finds none takes the tile kernel.
+// What the calling thread launches kernels with.  The workspace is its caller's -- a model's own buffer (its steps follow one another, so its
+// products can share it, replayed graphs included) or one made for a call -- with zeroed counters; without one, products that need it
+// take the tile kernel.
 struct LaunchScope {
   void* ws = nullptr;
   size_t bytes = 0;
@@ -826,25 +826,9 @@ bool launch_overlap() { return g_scope.overlap; }
 size_t rows_counter_bytes(int ctas) { return (static_cast<size_t>(ctas) * 4 * sizeof(unsigned int) + 1023) / 1024 * 1024; }
 size_t rows_slot_bytes(int tw, int mn) { return static_cast<size_t>(tw) * 128 * ((mn + 31) / 32 * 32) * sizeof(float); }
 
-void* rows_workspace(cudaStream_t stream, int ctas, int tw, int mn) {
+void* rows_workspace(int ctas, int tw, int mn) {
   const size_t need = rows_counter_bytes(ogb_num_sms()) + 2 * static_cast<size_t>(ctas) * rows_slot_bytes(tw, mn);
-  const size_t most = rows_counter_bytes(ogb_num_sms()) + 2 * static_cast<size_t>(ogb_num_sms()) * rows_slot_bytes(2, kRowsRangesM);
-  if (g_scope.ws != nullptr && g_scope.bytes >= need) return g_scope.ws;
-  static std::mutex mu;
-  static std::unordered_map<uint64_t, void*> table;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-  const uint64_t key = (static_cast<uint64_t>(dev) << 56) ^ reinterpret_cast<uint64_t>(stream);
-  std::lock_guard<std::mutex> lock(mu);
-  auto hit = table.find(key);
-  if (hit != table.end()) return hit->second;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return nullptr;
-  void* ws = nullptr;
-  if (cudaMalloc(&ws, most) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-  if (cudaMemset(ws, 0, rows_counter_bytes(ogb_num_sms())) != cudaSuccess) { cudaFree(ws); return nullptr; }
-  table.emplace(key, ws);
-  return ws;
+  return g_scope.bytes >= need ? g_scope.ws : nullptr;
 }
 
 template <int TW, int EPI>
@@ -864,7 +848,7 @@ static int launch_rows_one(const void* A, const void* W, int K, int lda, int ldw
     grid = sms;
     p.stages = std::min(kRowsMaxStages, (kRowsSmemMax - kRowsBarBytes - TW * kRowsStage) / stage_bytes);
     smem = p.stages * stage_bytes + kRowsBarBytes + TW * kRowsStage;
-    void* ws = rows_workspace(stream, grid, TW, p.mn);
+    void* ws = rows_workspace(grid, TW, p.mn);
     if (ws == nullptr) return kRowsDeclined;
     p.counters = static_cast<unsigned int*>(ws);
     p.ws = reinterpret_cast<float*>(static_cast<char*>(ws) + rows_counter_bytes(sms));
@@ -903,8 +887,8 @@ static int launch_rows(const void* A, const void* W, void* C, const void* bias, 
 
 using namespace ogb;
 
-// The buffer that products with few rows use when this thread launches them from now on (null: none).  It starts zeroed, holds
-// ogb_rows_workspace_bytes(rows) and serves one stream at a time.
+// The buffer that products with few rows use when this thread launches them from now on (null: none).  Its first ogb_rows_counter_bytes()
+// start zeroed; it holds ogb_rows_workspace_bytes(rows) and serves one stream at a time.
 // overlap: the kernels of a step may start before the one ahead of them has ended (see pdl_wait); every weight and every key of an
 // earlier step then has to be complete when the step begins.
 extern "C" void ogb_launch_scope(void* ws, int64_t bytes, int overlap) {
@@ -919,6 +903,7 @@ extern "C" int ogb_tile_sums(int on) {
   g_tile_sums = on != 0;
   return old;
 }
+extern "C" int64_t ogb_rows_counter_bytes(void) { return static_cast<int64_t>(rows_counter_bytes(ogb_num_sms())); }
 extern "C" int64_t ogb_rows_workspace_bytes(int rows) {
   const int mn = std::min(kRowsRangesM, (std::max(rows, 1) + 15) / 16 * 16);
   const int sms = ogb_num_sms();

@@ -533,7 +533,7 @@ static int launch_w4_rows_one(const void* x, int K, int ldx, RowsGemmParams p, W
     grid = sms;
     p.stages = std::min(kRowsMaxStages, (kRowsSmemMax - kRowsBarBytes - TW * kRowsStage) / stage_bytes);
     smem = p.stages * stage_bytes + kRowsBarBytes + TW * kRowsStage;
-    void* ws = rows_workspace(stream, grid, TW, p.mn);
+    void* ws = rows_workspace(grid, TW, p.mn);
     if (ws == nullptr) return kRowsDeclined;
     p.counters = static_cast<unsigned int*>(ws);
     p.ws = reinterpret_cast<float*>(static_cast<char*>(ws) + rows_counter_bytes(sms));
@@ -620,7 +620,7 @@ extern "C" int ogb_w4a16_gemm(const void* x, const void* qweight, const void* sc
 }
 
 // out[M, N / 2] = silu(gate) * up of a projection whose first N / 2 rows are the gate's and the others the up projection's; arguments as
-// above, without a bias.  M at most 256.  -11: not here (a capture outside a step has no workspace).
+// above, without a bias.  M at most 256.  -11: not here (more tiles than SMs, and no workspace or many rows).
 extern "C" int ogb_w4a16_gated(const void* x, const void* qweight, const void* scales, const void* zp, void* out, int M, int N, int K, int ldx, int ldc,
                                int scales_f32, int* status, void* stream_) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;

@@ -17,12 +17,14 @@ int ogb_num_sms(void);
 int ogb_gemm_bf16(const void* A, const void* W, void* C, const void* bias, const void* residual, void* C_f32, int M,
                   int N, int K, int lda, int ldw, int ldc, int ldr, int epilogue, int bn, int* status, void* stream);
 
-// Workspace that products with few rows use when the calling thread launches them from now on (null: one per stream): zeroed once,
-// ogb_rows_workspace_bytes(rows) bytes for products of up to `rows` rows, used on one stream at a time.  overlap != 0: kernels may start
+// Workspace that products with few rows use when the calling thread launches them from now on (null: none; those that need one then take
+// the tile kernel): its first ogb_rows_counter_bytes() zeroed once, ogb_rows_workspace_bytes(rows) bytes for products of up to `rows`
+// rows, used on one stream at a time.  overlap != 0: kernels may start
 // before the one ahead of them has ended, which wants every weight and every key of earlier steps complete when the step's first
 // kernel (the embedding) runs, and decode rows whose newest key alone is of this step.
 void ogb_launch_scope(void* ws, int64_t bytes, int overlap);
 int64_t ogb_rows_workspace_bytes(int rows);
+int64_t ogb_rows_counter_bytes(void);
 // on != 0: products that the calling thread launches from now on sum over K as the tile kernel alone does, whatever their rows (models
 // that choose among experts).  Returns the old setting.
 int ogb_tile_sums(int on);

@@ -240,19 +240,34 @@ def gemm(a, w, bias=None, residual=None, epilogue="none", out=None, out_f32=Fals
                                     a.stride(0), w.stride(0), out.stride(0), residual.stride(0) if residual is not None else 0,
                                     _EPI[epilogue], bn, a_ready[0], a_ready[1], a_ready[2], status_word().data_ptr(), _stream())
     else:
-        rc = lib.ogb_gemm_bf16(a.data_ptr(), w.data_ptr(), c_bf16, _ptr(bias), _ptr(residual), c_f32, m, n, k,
-                               a.stride(0), w.stride(0), out.stride(0), residual.stride(0) if residual is not None else 0,
-                               _EPI[epilogue], bn, status_word().data_ptr(), _stream())
+        with call_scope(m, -(-n_out // 128), a.device):
+            rc = lib.ogb_gemm_bf16(a.data_ptr(), w.data_ptr(), c_bf16, _ptr(bias), _ptr(residual), c_f32, m, n, k,
+                                   a.stride(0), w.stride(0), out.stride(0), residual.stride(0) if residual is not None else 0,
+                                   _EPI[epilogue], bn, status_word().data_ptr(), _stream())
     _native.check(rc, "ogb_gemm_bf16")
     launch_counts["gemm_bf16_tcgen05"] += 1
     return out
 
 
 def rows_workspace(rows: int, device) -> torch.Tensor:
-    """The zeroed buffer that products of up to ``rows`` rows keep partial sums in; see :func:`launch_scope`."""
+    """The buffer, its counters zeroed, that products of up to ``rows`` rows keep partial sums in; see :func:`launch_scope`."""
+    lib = _native.load()
     with torch.cuda.device(device):
-        n = _native.load().ogb_rows_workspace_bytes(int(rows))
-    return torch.zeros(n, dtype=torch.uint8, device=device)
+        n, counters = lib.ogb_rows_workspace_bytes(int(rows)), lib.ogb_rows_counter_bytes()
+    ws = torch.empty(n, dtype=torch.uint8, device=device)
+    ws[:counters].zero_()
+    return ws
+
+
+RANGES_MAX_M = 48       # rows up to which the products over more tiles than SMs come in ranges, which need a workspace
+
+
+def call_scope(m: int, tiles: int, device):
+    """A scope for one product of ``m`` rows over ``tiles`` tiles of its weight: the caller's, or where it has none and the product needs a
+    workspace, one that lives as long as the call (the allocator hands its memory on in the stream's order)."""
+    if getattr(_scopes, "now", None) is not None or m > RANGES_MAX_M or tiles <= torch.cuda.get_device_properties(device).multi_processor_count:
+        return contextlib.nullcontext()
+    return launch_scope(rows_workspace(m, device))
 
 
 _scopes = threading.local()      # .now: the (workspace, overlap) of the calling thread's innermost scope

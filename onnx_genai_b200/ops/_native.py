@@ -26,6 +26,7 @@ _SIGNATURES = {
     "ogb_gemm_bf16_wait": ([P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, P, P, ctypes.c_uint64, P, P], I),
     "ogb_launch_scope": ([P, L, I], None),
     "ogb_rows_workspace_bytes": ([I], L),
+    "ogb_rows_counter_bytes": ([], L),
     "ogb_tile_sums": ([I], I),
     "ogb_gemm_set_stream_k": ([I], I),
     "ogb_tp_set_pdl": ([I], I),
