@@ -14,6 +14,8 @@
 #include <cuda.h>
 #include <stdint.h>
 
+#include "per_device.h"
+
 namespace ogb {
 
 // Activations between the two products of a feed-forward.  Gated ones take a gate g and an up value u, the others one value v; a and b
@@ -243,6 +245,15 @@ inline cudaError_t launch_kernel_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 b
   cfg.attrs = pdl ? attr : nullptr;
   cfg.numAttrs = pdl ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// Lets a kernel have `bytes` of dynamic shared memory on the current device.
+template <typename Kernel>
+inline int allow_smem(OncePerDevice& once, Kernel kernel, int bytes) {
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  return once(device, [&] { return static_cast<int>(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)); });
 }
 
 template <typename... KArgs, typename... Args>

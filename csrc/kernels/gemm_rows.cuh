@@ -23,7 +23,7 @@
 
 #include <map>
 #include <mutex>
-#include <utility>
+#include <tuple>
 
 #include "gemm_common.cuh"
 
@@ -64,11 +64,13 @@ size_t rows_counter_bytes(int ctas);
 template <typename Kernel>
 static int rows_pick_splits(Kernel kernel, int threads, int smem, int tiles, int k_blocks) {
   static std::mutex mu;
-  static std::map<std::pair<const void*, int>, int> most;        // (kernel, shared memory and split) -> clusters at once
+  static std::map<std::tuple<int, const void*, int>, int> most;  // (device, kernel, shared memory and split) -> clusters at once
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) { cudaGetLastError(); return 1; }
   std::lock_guard<std::mutex> lock(mu);
   for (int s = kRowsMaxSplit; s > 1; --s) {
     if (2 * s > k_blocks) continue;
-    const std::pair<const void*, int> key(reinterpret_cast<const void*>(kernel), smem * 16 + s);
+    const std::tuple<int, const void*, int> key(device, reinterpret_cast<const void*>(kernel), smem * 16 + s);
     auto hit = most.find(key);
     if (hit == most.end()) {
       cudaLaunchConfig_t cfg = {};

@@ -834,11 +834,9 @@ void* rows_workspace(int ctas, int tw, int mn) {
 template <int TW, int EPI>
 static int launch_rows_one(const void* A, const void* W, int K, int lda, int ldw, RowsGemmParams p, const ActArgs& act, cudaStream_t stream) {
   auto kernel = gemm_rows_kernel<TW, EPI>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    OGB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmemMax));
-    attr_set = true;
-  }
+  static OncePerDevice allowed;
+  int rc = allow_smem(allowed, kernel, kRowsSmemMax);
+  if (rc != 0) return rc;
   const int sms = ogb_num_sms();
   const int stage_bytes = TW * 128 * kBK * 2 + p.mn * kBK * 2;
   p.n_tiles = (p.N + TW * 128 - 1) / (TW * 128);
@@ -861,7 +859,7 @@ static int launch_rows_one(const void* A, const void* W, int K, int lda, int ldw
     grid = p.n_tiles * p.splits;
   }
   CUtensorMap mw, ma;
-  int rc = make_tmap_bf16_2d(&mw, W, p.N, K, ldw, 128, kBK);
+  rc = make_tmap_bf16_2d(&mw, W, p.N, K, ldw, 128, kBK);
   if (rc != 0) return rc;
   rc = make_tmap_bf16_2d(&ma, A, p.M, K, lda, p.mn, kBK);
   if (rc != 0) return rc;

@@ -518,11 +518,9 @@ gemm_w4_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const RowsGemmPa
 template <int TW, int EPI, bool SF32>
 static int launch_w4_rows_one(const void* x, int K, int ldx, RowsGemmParams p, W4RowsParams wp, cudaStream_t stream) {
   auto kernel = gemm_w4_rows_kernel<TW, EPI, SF32>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    OGB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmemMax));
-    attr_set = true;
-  }
+  static OncePerDevice allowed;
+  int rc = allow_smem(allowed, kernel, kRowsSmemMax);
+  if (rc != 0) return rc;
   const int sms = ogb_num_sms();
   const int stage_bytes = TW * kWTile * kWBK * 2 + p.mn * kWBK * 2;
   p.n_tiles = (wp.tile_rows + kWTile - 1) / kWTile;
@@ -544,7 +542,7 @@ static int launch_w4_rows_one(const void* x, int K, int ldx, RowsGemmParams p, W
     grid = p.n_tiles * p.splits;
   }
   CUtensorMap ta;
-  const int rc = make_tmap_bf16_2d(&ta, x, p.M, K, ldx, p.mn, kWBK);
+  rc = make_tmap_bf16_2d(&ta, x, p.M, K, ldx, p.mn, kWBK);
   if (rc != 0) return rc;
   return rows_launch(kernel, grid, kWThreads, smem, p.splits, stream, ta, p, wp, ActArgs());
 }

@@ -433,12 +433,9 @@ inline int launch_sample_cluster(const void* logits, int* out, const float* temp
                                  const float* uniform, int rows, int vocab, int ld, cudaStream_t stream) {
   const int slice = ((vocab + kClCtas - 1) / kClCtas + 7) / 8 * 8;
   const int smem = static_cast<int>((sizeof(ClShared) + 15) / 16 * 16) + slice * 2;
-  static bool attr_set = false;
-  if (!attr_set) {
-    OGB_CUDA_CHECK(cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>((sizeof(ClShared) + 15) / 16 * 16) + kClMaxSlice * 2));
-    attr_set = true;
-  }
+  static OncePerDevice allowed;
+  const int rc = allow_smem(allowed, sample_cluster_kernel, static_cast<int>((sizeof(ClShared) + 15) / 16 * 16) + kClMaxSlice * 2);
+  if (rc != 0) return rc;
   sample_cluster_kernel<<<rows * kClCtas, kClThreads, smem, stream>>>(static_cast<const __nv_bfloat16*>(logits), out, temperature, top_k, top_p, min_p,
                                                                       uniform, vocab, ld, slice);
   return static_cast<int>(cudaGetLastError());
