@@ -22,6 +22,7 @@ constexpr int kClThreads = 512;
 constexpr int kClWarps = kClThreads / 32;
 constexpr int kClBuckets = 1024;
 constexpr int kClList = 1024;
+constexpr int kClMaxCuts = 3;                // a cut leaves a 1024th of the range of weights: 2^30 values, 2^20, 2^10, 1
 constexpr uint32_t kClLow = 1u << 16;        // smaller weights are summed, and looked at one by one only where a threshold falls among them
 constexpr int kClMaxSlice = 65536;           // logits per CTA: 2^16 low halves of weights still sum below 2^32
 
@@ -269,7 +270,7 @@ sample_cluster_kernel(const __nv_bfloat16* __restrict__ logits, int* __restrict_
       if (above + (by_mass ? rest_mass : rest_cnt) < target) return floor_w;
       to = kClLow - 1;
     }
-    for (;;) {
+    for (int cuts = 0; cuts <= kClMaxCuts; ++cuts) {
       if (tid == 0) { sh.n = 0; sh.w_min = 0xffffffffu; sh.w_max = 0u; sh.thr = 0u; }
       __syncthreads();
       for (int vi = tid; vi < nvec; vi += kClThreads)
@@ -333,6 +334,7 @@ sample_cluster_kernel(const __nv_bfloat16* __restrict__ logits, int* __restrict_
       from = w_min + static_cast<uint32_t>((c * width + kClBuckets - 1) / kClBuckets);
       to = w_min + static_cast<uint32_t>(((c + 1) * width + kClBuckets - 1) / kClBuckets) - 1;
     }
+    return from;                                                   // not reached: after kClMaxCuts one weight is left
   };
   // summed weight of this thread's tokens in vectors [v0, v1), v0 + step, ... with weights of at least thr
   auto mass_of = [&](int v0, int v1, int step, uint32_t thr) {
