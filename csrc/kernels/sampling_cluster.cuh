@@ -32,7 +32,7 @@ struct ClShared {
   unsigned long long row_mass[kClBuckets];
   uint32_t list[kClList], cand[kClList];
   float high[kClWarps], low[kClWarps];
-  unsigned long long sums[32];
+  unsigned long long sums[kClWarps], scan[kClWarps];             // cl_block_sum's; find's, written while a slower warp may still read the other
   // one slot per exchange with the other CTAs that can be under way while a slower CTA still reads the last one
   float best, lowest;
   int first;
@@ -207,10 +207,10 @@ sample_cluster_kernel(const __nv_bfloat16* __restrict__ logits, int* __restrict_
       if (lane >= o) incl += n;
     }
     if (tid == 0) sh.bucket = -1;
-    if (lane == 31) sh.sums[warp] = incl;
+    if (lane == 31) sh.scan[warp] = incl;
     __syncthreads();
     unsigned long long run = above + incl - a - b;
-    for (int i = 0; i < warp; ++i) run += sh.sums[i];
+    for (int i = 0; i < warp; ++i) run += sh.scan[i];
     if (run < target && run + a >= target) { sh.bucket = 2 * tid; sh.above = run; }
     run += a;
     if (run < target && run + b >= target) { sh.bucket = 2 * tid + 1; sh.above = run; }

@@ -20,3 +20,12 @@ def test_cuts_end():
             assert all(-(-(c + 1) * width // n) - -(-c * width // n) <= widest for c in probe)
             width, cuts = widest, cuts + 1
         assert cuts <= _constant("kClMaxCuts")
+
+
+def test_sums_and_searches_write_words_of_their_own():
+    """cl_block_sum ends in reads without a barrier behind them, so what comes next must not write the same words: a search may come next."""
+    search = SOURCE[SOURCE.index("auto find = "):]
+    search = search[:search.index("\n  };")]
+    assert "sh.sums" not in search
+    uses = [m.start() for m in re.finditer(r"sh\.sums\[warp\] = ", SOURCE)]
+    assert all("__syncthreads();" in SOURCE[at - 120:at] for at in uses)       # the others wait for the reads first
