@@ -259,6 +259,13 @@ def rows_workspace(rows: int, device) -> torch.Tensor:
     return ws
 
 
+def in_order():
+    """Inside a scope whose kernels start early, none for those launched here: each starts when the one ahead of it has ended, as a product
+    must whose weight an earlier kernel of the same step writes."""
+    scope = getattr(_scopes, "now", None)
+    return launch_scope(scope[0]) if scope is not None and scope[1] else contextlib.nullcontext()
+
+
 RANGES_MAX_M = 48       # rows up to which the products over more tiles than SMs come in ranges, which need a workspace
 
 

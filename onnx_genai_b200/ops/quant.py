@@ -5,7 +5,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _native, call_scope, launch_counts, reference, status_word, timed_region
+from . import _native, call_scope, in_order, launch_counts, reference, status_word, timed_region
 from . import gemm as _gemm
 
 GEMV_MAX_M = 8          # rows the GEMV kernels accept
@@ -146,6 +146,8 @@ class QuantLinear:
                                            self._scratch.data_ptr(), self.n, self.k, int(self.scales_fp32), stream)
             _native.check(rc, "ogb_w4a16_dequant")
             launch_counts["w4a16_dequant"] += 1
+            with in_order():                       # the weight is not complete before that kernel has ended
+                return _gemm(x, self._scratch, bias=self.bias, out=out)
         return _gemm(x, self._scratch, bias=self.bias, out=out)
 
     def device_weight_bytes(self) -> int:

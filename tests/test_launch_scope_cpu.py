@@ -66,3 +66,14 @@ def test_sums_by_tiles_nest(library):
             assert not library.sums
         assert library.sums
     assert not library.sums
+
+
+def test_kernels_in_order_inside_a_scope(library):
+    with ops.in_order():
+        pass
+    assert not library.calls                      # outside a scope nothing starts early
+    ws = torch.zeros(64, dtype=torch.uint8)
+    with ops.launch_scope(ws, True):
+        with ops.in_order():
+            assert _last(library) == (ws.data_ptr(), 64, 0)
+        assert _last(library) == (ws.data_ptr(), 64, 1)
