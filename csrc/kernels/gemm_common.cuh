@@ -44,10 +44,11 @@ OGB_DEVICE float plain_act(const ActArgs& act, float v) {
 // finisher, which always has the higher block index, waits for those flags (bounded) and adds the partials before
 // its epilogue.  Waiting only on lower-numbered CTAs keeps the scheme free of deadlock whatever the residency, and
 // walking every range backwards (GemmWork::next) makes partials the first thing a CTA produces and fix-ups the last.
-// With more tiles than CTAs only those of about the last wave are cut (sk_cut_tiles), and they come first: the whole waves that follow
+// With more tiles than CTAs only those of about the last wave are cut (sk_cut_tiles in gemm_plan.h), and they come first: the whole waves that follow
 // are dealt round-robin, so that CTAs walk K in step and share what they read through L2 (cut from end to end, 7100 rows
 // against a 3584 x 18944 projection drew every operand from HBM again and again: 1101 us), and a fix-up's wait passes
-// under the main loop of the tile after it.  Where the order of the sums must stay (tile_sums), all tiles are cut.
+// under the main loop of the tile after it.  Where the order of the sums must stay (tile_sums) and in the scatter epilogue of the
+// tensor-parallel path, whose tiles arrive at other GPUs in the order of the ranges, all tiles are cut.
 // ----------------------------------------------------------------------------------------
 // Tiles of many rows: 16 tiles of A at a time against every tile of W, so that the tiles under way at one moment (about 148) span
 // 2048 rows of A and 2400 of W instead of all of A and two tiles of W.
@@ -65,14 +66,6 @@ OGB_DEVICE void raster_tile(int tile, int m_tiles, int n_tiles, bool grouped, in
   const int rows = min(kRasterM, m_tiles - first), t = tile - first * n_tiles;
   mt = first + t % rows;
   nt = t / rows;
-}
-
-// How many of a launch's first tiles stream-K cuts into ranges: all when there are fewer than CTAs, else those of the incomplete last wave,
-// and a wave more where they are so few that many CTAs would share each of them.
-inline int sk_cut_tiles(int tiles, int ctas) {
-  if (tiles <= ctas) return tiles;
-  const int rest = tiles % ctas;
-  return 2 * ctas > 7 * rest ? rest + ctas : rest;
 }
 
 struct GemmSeg {

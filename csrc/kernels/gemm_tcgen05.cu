@@ -26,6 +26,7 @@
 
 #include "common.cuh"
 #include "gemm_common.cuh"
+#include "gemm_plan.h"
 #include "gemm_rows.cuh"
 #include "ogb_kernels.h"
 #include "tp_comm.cuh"
@@ -710,53 +711,6 @@ static bool stream_k_enabled() {
   }
   return g_stream_k == 1;
 }
-// Stream-K pays when round-robin tiles would leave a large part of the last wave idle and the fix-up is cheap next
-// to a tile: every CTA boundary that falls inside a tile costs one fp32 partial written and read back and a flag wait
-// in the finisher.  `fix` is that cost in k-blocks of tensor-core time.  Measured on the 7B shapes (tile widths 32 - 256
-// with and without stream-K, M = 32 - 1472): about 40 for a plain epilogue -- with 13 the estimate chose wide stream-K
-// tiles for K = 3584 projections that ran 1.3 - 1.5x slower than plain 128-wide tiles -- while the scatter epilogue of
-// the tensor-parallel path, whose tiles end in stores to other GPUs, keeps the 13 it was tuned with.
-constexpr float kSkFixPlain = 40.0f;
-constexpr float kSkFixScatter = 13.0f;
-// A finisher adds the partials of a tile one after the other, so the fix-up grows with the CTAs that share a tile once they are many
-// (8 tiles on 148 SMs, 19 each, took 123 us where whole tiles take 20).
-constexpr float kSkShared = 6.0f;
-// With whole waves after the cut tiles (sk_cut_tiles) the fix-ups pass under the main loops of the tiles after them, as long as those
-// are long enough.  A CTA's partial costs about 25 k-blocks to write and add (0.3 us each at 256 columns): 7100 and 2304 rows against
-// 3584 x 18944 gain 1244 -> 690 and 298 -> 234 us; with K = 3584 (2304 rows: 54 -> 71 us) the fix-ups are what is left.
-constexpr float kSkPartial = 25.0f;
-// A launch's rule: the fix-up's cost, and whether all tiles are cut.
-struct SkRule {
-  float fix;
-  bool all;
-  int cut(int tiles, int sms) const { return all ? tiles : sk_cut_tiles(tiles, sms); }
-};
-// The cost of the fix-ups of a launch, in k-blocks.
-static float sk_fix(int tiles, int k_blocks, int sms, SkRule rule) {
-  const float fix = rule.fix;
-  const int cut = rule.cut(tiles, sms);
-  const float shared = static_cast<float>(sms) / static_cast<float>(std::max(cut, 1));
-  if (cut < tiles) {
-    const float own = kSkPartial * (1.f + shared);
-    return own < 0.5f * static_cast<float>(k_blocks) ? 0.25f * own : 1e6f;
-  }
-  return shared > kSkShared ? fix * shared / kSkShared : fix;
-}
-static bool stream_k_applies(int tiles, int k_blocks, int sms, SkRule rule) {
-  if (!stream_k_enabled() || tiles % sms == 0 || static_cast<long long>(tiles) * k_blocks < 2LL * sms) return false;
-  const float w = static_cast<float>(tiles) / static_cast<float>(sms);
-  const float dp = static_cast<float>((tiles + sms - 1) / sms);
-  const float sk = w + sk_fix(tiles, k_blocks, sms, rule) / static_cast<float>(k_blocks);
-  return sk < 0.93f * dp;
-}
-// Relative duration of a launch with `tiles` tiles of relative cost `cost`: whole waves when tiles are dealt
-// round-robin, the exact share plus the fix-up when stream-K spreads the k-blocks evenly.
-static float launch_cost(int tiles, int k_blocks, int sms, float cost, SkRule rule) {
-  if (stream_k_applies(tiles, k_blocks, sms, rule))
-    return (static_cast<float>(tiles) / static_cast<float>(sms) + sk_fix(tiles, k_blocks, sms, rule) / static_cast<float>(k_blocks)) * cost;
-  return static_cast<float>((tiles + sms - 1) / sms) * cost;
-}
-
 template <int BN, int EPI>
 static int launch_gemm(const void* A, const void* W, void* C, const void* bias, const void* residual, void* C_f32, int M,
                        int N, int K, int lda, int ldw, int ldc, int ldr, int* status, cudaStream_t stream,
@@ -786,8 +740,8 @@ static int launch_gemm(const void* A, const void* W, void* C, const void* bias, 
   uint32_t* sk_flags = nullptr;
   uint32_t sk_seq = 0;
   const int k_blocks = (K + kBK - 1) / kBK;
-  batch.raster = group_tab == nullptr && batch.count == 1 && !tile_sums() && static_cast<long long>(M) * K * 2 > kRasterBytes;
-  const SkRule rule{EPI == kEpiScatter ? kSkFixScatter : kSkFixPlain, tile_sums()};
+  const SkRule rule = sk_rule(EPI == kEpiScatter, tile_sums(), stream_k_enabled());
+  batch.raster = group_tab == nullptr && batch.count == 1 && !rule.all && static_cast<long long>(M) * K * 2 > kRasterBytes;
   if (group_tab == nullptr && stream_k_applies(tiles, k_blocks, sms, rule)) {
     SkWorkspace* w = sk_workspace(stream, sms);
     if (w != nullptr) {
@@ -978,7 +932,7 @@ static int gemm_bf16_dispatch(const void* A, const void* W, void* C, const void*
     for (int i = 0; i < 5; ++i) {
       if (cand[i] < 128 && m_tiles > 3) break;  // narrow tiles only pay off for decode-sized M
       const int tiles = m_tiles * ((N + cand[i] - 1) / cand[i]) * batch.count;
-      const float t = launch_cost(tiles, (K + kBK - 1) / kBK, sms, cost[i], SkRule{kSkFixPlain, tile_sums()});
+      const float t = launch_cost(tiles, (K + kBK - 1) / kBK, sms, cost[i], sk_rule(false, tile_sums(), stream_k_enabled()));
       if (t < best - 1e-6f) { best = t; bn = cand[i]; }
     }
   }
@@ -1055,7 +1009,7 @@ extern "C" int ogb_gemm_bf16_scatter(const void* A, const void* W, int M, int N,
     bn = 256;
     for (int i = 0; i < 3; ++i) {
       const int tiles = m_tiles * ((N + cand[i] - 1) / cand[i]);
-      const float t = launch_cost(tiles, (K + kBK - 1) / kBK, sms, cost[i], SkRule{kSkFixScatter, tile_sums()});
+      const float t = launch_cost(tiles, (K + kBK - 1) / kBK, sms, cost[i], sk_rule(true, tile_sums(), stream_k_enabled()));
       if (t < best - 1e-6f) { best = t; bn = cand[i]; }
     }
   }
