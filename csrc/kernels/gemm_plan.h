@@ -61,4 +61,43 @@ inline float launch_cost(int tiles, int k_blocks, int sms, float cost, const SkR
   return static_cast<float>((tiles + sms - 1) / sms) * cost;
 }
 
+// ----------------------------------------------------------------------------------------
+// Products with few rows (gemm_rows.cuh), or the tile kernel.  All times in us on B200, weights from HBM, tile kernel -> few rows.
+// ----------------------------------------------------------------------------------------
+constexpr int kRowsMaxM = 256;              // rows of the activation tile (the MMA's N)
+constexpr int kRowsGatedM = 32;             // of a gated product's
+constexpr int kRowsRangesM = 48;            // of one over more tiles than SMs
+
+// Rows up to which a product over `tiles` tiles of 128 columns (of 128 gate and 128 up columns, when gated) comes to the kernels for few rows.
+inline int rows_limit(int tiles, int k_blocks, bool gated, bool residual, int sms) {
+  if (tiles > sms) {
+    // ranges: a tile's epilogue has to pass under the k-blocks of the others, so a range needs enough of them.  N x K at 1 row: 152064 x 3584
+    // 225 -> 170, 151936 x 896 79 -> 70, 32000 x 2048 40 -> 39, but 32000 x 896 24 -> 29, 20000 x 576 16 -> 23, and with tiles of 9 k-blocks
+    // 151936 x 576 51 -> 57 at 16 rows; at 48: 151936 x 2048 126 -> 125, 65536 x 2048 65 -> 70, 151936 x 896 68 -> 76.
+    const long long blocks = static_cast<long long>(tiles) * k_blocks * (gated ? 2 : 1);
+    if (k_blocks < 12 || blocks < 52LL * sms) return 0;
+    return blocks < 150LL * sms || gated ? kRowsGatedM : kRowsRangesM;
+  }
+  // One CTA or a cluster per tile.  The tile kernel reads 128 rows of activations for each of its tiles, this one as many as there are, so the line
+  // falls with the rows; and it falls with the tiles, as fewer CTAs share a tile and more of the chip is busy in the tile kernel too.
+  if (tiles > sms / 2) {
+    // a CTA per tile: 16640 x 3584 42 -> 35 at 1 row, 37 -> 37 at 48, 38 -> 42 at 128; 9600 x 2048 26 -> 21, 22 -> 23, 22 -> 27; gated 37888 x 3584
+    // 57 -> 49 at 16, 37888 x 2048 44 -> 43 at 16, 42 -> 45 at 32
+    if (gated) return k_blocks >= 48 ? kRowsGatedM : 16;
+    return k_blocks >= 48 ? 48 : 32;
+  }
+  if (gated) return kRowsGatedM;
+  if (3 * tiles > sms) {
+    // two: 7168 x 2048 22 -> 19 at 1 row, 20 -> 19 at 48, 19 -> 21 at 64; x 3584 27 -> 27 at 128, 29 -> 31 at 200; x 8192 52 -> 53 at 256
+    return k_blocks >= 96 ? kRowsMaxM : k_blocks >= 48 ? 128 : 48;
+  }
+  // three to eight: 4608 x 3584 27 -> 13 at 1 row, 22 -> 19 at 256; 3584 x 18944 86 -> 31, 110 -> 48; 3584 x 2048 18 -> 19 at 128, 18 -> 21 at 256;
+  // 3584 x 896 13 -> 13 at 64, 12 -> 14 at 128.  With a residual all of them: the sum with it is rounded once here, twice in the tile kernel.
+  return residual || k_blocks >= 48 ? kRowsMaxM : k_blocks >= 24 ? 128 : 64;
+}
+inline bool rows_applies(int m, int n, int k_blocks, bool gated, bool residual, int sms) {
+  const int width = gated ? 256 : 128;
+  return m <= rows_limit((n + width - 1) / width, k_blocks, gated, residual, sms);
+}
+
 }  // namespace ogb

@@ -17,7 +17,7 @@
 // epilogue stores took longer than the products from 64 rows on.
 // TW = 2 takes 128 gate rows of W and their 128 up rows per tile (two accumulators): a packed gated projection, 128 columns of C.
 //
-// Measured on B200 (weights not in L2): see the dispatch rule in gemm_tcgen05.cu.
+// Measured on B200 (weights not in L2): see the rule in gemm_plan.h.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -26,6 +26,7 @@
 #include <tuple>
 
 #include "gemm_common.cuh"
+#include "gemm_plan.h"
 
 namespace ogb {
 
@@ -33,8 +34,6 @@ constexpr int kRowsThreads = 192;
 constexpr int kRowsMaxStages = 12;
 constexpr int kRowsSmemMax = 227 * 1024;
 constexpr int kRowsBarBytes = 512;
-constexpr int kRowsMaxM = 256;              // rows of the activation tile (the MMA's N)
-constexpr int kRowsGatedM = 32, kRowsRangesM = 48;   // rows up to which the other forms come here (dispatch in gemm_tcgen05.cu)
 constexpr int kRowsMaxSplit = 8;            // the portable cluster size
 constexpr int kRowsStage = 32 * 128 * 4;    // staging of 32 result rows of an accumulator (ranges)
 

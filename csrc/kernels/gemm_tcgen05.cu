@@ -855,6 +855,11 @@ extern "C" int ogb_tile_sums(int on) {
   g_tile_sums = on != 0;
   return old;
 }
+// 1: a product of these sizes (gated: over N gate and up columns together) sums in ranges and takes a workspace.
+extern "C" int ogb_rows_in_ranges(int M, int N, int K, int gated) {
+  const int sms = ogb_num_sms(), width = gated != 0 ? 256 : 128;
+  return !tile_sums() && (N + width - 1) / width > sms && rows_applies(M, N, (K + kBK - 1) / kBK, gated != 0, false, sms) ? 1 : 0;
+}
 extern "C" int64_t ogb_rows_counter_bytes(void) { return static_cast<int64_t>(rows_counter_bytes(ogb_num_sms())); }
 extern "C" int64_t ogb_rows_workspace_bytes(int rows) {
   const int mn = std::min(kRowsRangesM, (std::max(rows, 1) + 15) / 16 * 16);
@@ -905,14 +910,10 @@ static int gemm_bf16_dispatch(const void* A, const void* W, void* C, const void*
   if (epilogue == kEpiResidual && (residual == nullptr || (ldr % 8) != 0)) return -5;
   if (epilogue == kEpiSwiGLU && (bn < 64 || (N % bn) != 0 || C_f32 != nullptr)) return -6;
   if (batch.count < 1 || (batch.a_step % 8) != 0 || (batch.c_step % 8) != 0 || (batch.count > 1 && (a_ready != nullptr || epilogue != kEpiNone))) return -9;
-  // Few rows: gemm_rows.cuh.  Where the line lies, in us on B200 with weights from HBM, tile kernel -> this one (floor):
-  //   tiles of 128 columns for at most one wave, clusters over K: better at all sizes it takes.  N x K = 4608 x 3584 (5): 26.7 -> 12.9 at 1
-  //     row, 21.5 -> 18.9 at 256; 3584 x 18944 (21): 85.9 -> 31.4, 110 -> 48.0; 128 x 2048: 12.4 -> 7.1, 12.7 -> 11.7
-  //   more tiles, ranges: 152064 x 3584 (169): 225 -> 170 at 1 row, 185 -> 177 at 40, 188 -> 184 at 77, 193 -> 200 at 128; 151936 x 896 (42):
-  //     65 -> 53, 66 -> 63, 54 -> 71, 58 -> 84: the epilogue of a tile is as long as its few k-blocks
-  //   gated 37888 x 3584 (42): 57 -> 49 at 16, 49.2 -> 50.0 at 40, 49.6 -> 53.2 at 77: one tile per SM, whose epilogue nothing hides
-  const int rows_max = epilogue == kEpiSwiGLU ? kRowsGatedM : (N + 127) / 128 > ogb_num_sms() ? kRowsRangesM : kRowsMaxM;
-  if (M <= rows_max && !tile_sums() && a_ready == nullptr && batch.count == 1 && batch.page_d == 0 && (epilogue == kEpiSwiGLU ? bn == 256 : bn == 0)) {
+  // Few rows: gemm_rows.cuh (gemm_plan.h says where they end).
+  const bool gated = epilogue == kEpiSwiGLU;
+  if (!tile_sums() && a_ready == nullptr && batch.count == 1 && batch.page_d == 0 && (gated ? bn == 256 : bn == 0) &&
+      rows_applies(M, N, (K + kBK - 1) / kBK, gated, epilogue == kEpiResidual, ogb_num_sms())) {
     const int rc = launch_rows(A, W, C, bias, residual, C_f32, M, N, K, lda, ldw, ldc, ldr, epilogue, act, status, stream);
     if (rc != kRowsDeclined) return rc;
   }

@@ -25,6 +25,8 @@ int ogb_gemm_bf16(const void* A, const void* W, void* C, const void* bias, const
 void ogb_launch_scope(void* ws, int64_t bytes, int overlap);
 int64_t ogb_rows_workspace_bytes(int rows);
 int64_t ogb_rows_counter_bytes(void);
+// 1: a product of these sizes (gated: N gate and up columns together) takes a workspace.
+int ogb_rows_in_ranges(int M, int N, int K, int gated);
 // on != 0: products that the calling thread launches from now on sum over K as the tile kernel alone does, whatever their rows (models
 // that choose among experts).  Returns the old setting.
 int ogb_tile_sums(int on);

@@ -240,7 +240,7 @@ def gemm(a, w, bias=None, residual=None, epilogue="none", out=None, out_f32=Fals
                                     a.stride(0), w.stride(0), out.stride(0), residual.stride(0) if residual is not None else 0,
                                     _EPI[epilogue], bn, a_ready[0], a_ready[1], a_ready[2], status_word().data_ptr(), _stream())
     else:
-        with call_scope(m, -(-n_out // 128), a.device):
+        with call_scope(m, lambda: lib.ogb_rows_in_ranges(m, n, k, int(epilogue == "swiglu")), a.device):
             rc = lib.ogb_gemm_bf16(a.data_ptr(), w.data_ptr(), c_bf16, _ptr(bias), _ptr(residual), c_f32, m, n, k,
                                    a.stride(0), w.stride(0), out.stride(0), residual.stride(0) if residual is not None else 0,
                                    _EPI[epilogue], bn, status_word().data_ptr(), _stream())
@@ -266,15 +266,15 @@ def in_order():
     return launch_scope(scope[0]) if scope is not None and scope[1] else contextlib.nullcontext()
 
 
-RANGES_MAX_M = 48       # rows up to which the products over more tiles than SMs come in ranges, which need a workspace
+RANGES_MAX_M = 48       # rows of the products that need a workspace, at most
 
 
-def call_scope(m: int, tiles: int, device):
-    """A scope for one product of ``m`` rows over ``tiles`` tiles of its weight: the caller's, or where it has none and the product needs a
-    workspace, one that lives as long as the call (the allocator hands its memory on in the stream's order)."""
-    if getattr(_scopes, "now", None) is not None or m > RANGES_MAX_M or tiles <= torch.cuda.get_device_properties(device).multi_processor_count:
+def call_scope(rows: int, in_ranges, device):
+    """A scope for one product: the caller's, or where it has none and ``in_ranges()`` says that the product needs a workspace, one that
+    lives as long as the call (the allocator hands its memory on in the stream's order)."""
+    if getattr(_scopes, "now", None) is not None or rows > RANGES_MAX_M or not in_ranges():
         return contextlib.nullcontext()
-    return launch_scope(rows_workspace(m, device))
+    return launch_scope(rows_workspace(rows, device))
 
 
 _scopes = threading.local()      # .now: the (workspace, overlap) of the calling thread's innermost scope

@@ -27,6 +27,7 @@ _SIGNATURES = {
     "ogb_launch_scope": ([P, L, I], None),
     "ogb_rows_workspace_bytes": ([I], L),
     "ogb_rows_counter_bytes": ([], L),
+    "ogb_rows_in_ranges": ([I, I, I, I], I),
     "ogb_tile_sums": ([I], I),
     "ogb_gemm_set_stream_k": ([I], I),
     "ogb_tp_set_pdl": ([I], I),

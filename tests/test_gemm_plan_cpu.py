@@ -67,3 +67,52 @@ def test_other_products_cut_the_last_wave(plan):
         waves = -(-tiles // 148)
         assert cost <= waves and (on or cost == waves)
     assert not any(on for on, _, _ in plan([(0, 0, 0, t, kb, 148) for t, kb in SIZES]))
+
+
+ROWS = r"""
+#include <cstdio>
+#include "gemm_plan.h"
+int main() {
+  int m, n, kb, gated, residual, sms;
+  while (std::scanf("%d %d %d %d %d %d", &m, &n, &kb, &gated, &residual, &sms) == 6)
+    std::printf("%d\n", ogb::rows_applies(m, n, kb, gated, residual, sms) ? 1 : 0);
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def rows(tmp_path_factory):
+    if shutil.which("g++") is None:
+        pytest.skip("needs g++")
+    d = tmp_path_factory.mktemp("rows")
+    (d / "main.cpp").write_text(ROWS)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(KERNELS), str(d / "main.cpp"), "-o", str(d / "main")], check=True)
+
+    def ask(m, n, k, gated, residual=False):
+        out = subprocess.run([str(d / "main")], input=f"{m} {n} {-(-k // 64)} {int(gated)} {int(residual)} 148", capture_output=True, text=True, check=True).stdout
+        return out.strip() == "1"
+
+    return ask
+
+
+# (rows, N, K, gated): where the kernels for few rows took 1.1 to 1.65 times the tile kernel's time, and where they took 0.4 to 0.9 of it
+SLOWER = [(256, 7168, 896, False), (256, 16640, 896, False), (256, 9600, 2048, False), (128, 9600, 896, False), (256, 9600, 3584, False), (128, 3584, 896, False),
+          (256, 18944, 8192, False), (64, 18944, 896, False), (1, 20000, 576, False), (48, 20000, 896, False), (16, 32000, 896, False), (48, 65536, 2048, False),
+          (16, 151936, 576, False), (48, 151936, 896, False), (16, 49152, 896, True), (32, 37888, 2048, True)]
+FASTER = [(1, 128, 2048, False), (256, 4608, 3584, False), (256, 3584, 18944, False), (64, 7168, 18944, False), (1, 18944, 3584, False), (16, 9600, 2048, False),
+          (1, 152064, 3584, False), (48, 152064, 3584, False), (1, 151936, 896, False), (16, 128256, 2048, False), (32, 9728, 4096, True), (16, 37888, 3584, True),
+          (8, 49152, 4096, True)]
+
+
+@pytest.mark.parametrize("size", SLOWER)
+def test_few_rows_are_left_to_the_tile_kernel_where_it_is_faster(rows, size):
+    assert not rows(*size)
+
+
+@pytest.mark.parametrize("size", FASTER)
+def test_few_rows_have_their_own_kernel_where_that_is_faster(rows, size):
+    assert rows(*size)
+
+
+def test_sums_with_a_residual_stay_where_they_are_rounded_once(rows):
+    assert all(rows(256, n, k, False, True) for n, k in [(128, 64), (3584, 512), (896, 896), (4608, 18944)])

@@ -4,14 +4,16 @@ import pytest
 import torch
 
 from onnx_genai_b200 import ops
+from onnx_genai_b200.ops import _native
 
 pytestmark = pytest.mark.gpu
 
 
-def _operands(m, n, k=448):
+def _operands(m, n, k=3592):
     g = torch.Generator(device="cuda").manual_seed(m + n)
     a = torch.randn(m, k, device="cuda", generator=g).bfloat16()
     w = (torch.randn(n, k, device="cuda", generator=g) * 0.05).bfloat16()
+    assert _native.load().ogb_rows_in_ranges(m, n, k, 0)
     with ops.launch_scope(ops.rows_workspace(m, "cuda")):
         return a, w, ops.gemm(a, w)
 
@@ -36,7 +38,7 @@ def test_streams_of_their_own():
 
 
 def test_a_graph_beside_the_stream_that_it_was_captured_on():
-    a, w, want = _operands(33, 19000)
+    a, w, want = _operands(32, 19000)
     side, other = torch.cuda.Stream(), torch.cuda.Stream()
     with torch.cuda.stream(side):
         ops.gemm(a, w)
