@@ -17,8 +17,12 @@ constexpr float kSkFixScatter = 13.0f;
 constexpr float kSkShared = 6.0f;
 // With whole waves after the cut tiles (sk_cut_tiles) the fix-ups pass under the main loops of the tiles after them, as long as those
 // are long enough.  A CTA's partial costs about 25 k-blocks to write and add (0.3 us each at 256 columns): 7100 and 2304 rows against
-// 3584 x 18944 gain 1244 -> 690 and 298 -> 234 us; with K = 3584 (2304 rows: 54 -> 71 us) the fix-ups are what is left.
+// 3584 x 18944 gain 1244 -> 690 and 298 -> 234 us; with K = 3584 (2304 rows: 54 -> 71 us) the fix-ups are what is left.  Where the main
+// loops are too short for that, all tiles of 256 columns may be cut, as long as W stays in L2 for the CTAs that read it out of step: 4096 rows
+// against 3584 x 5120 (37 MB) 146 us in whole tiles, 125 so; 7100 against 2048 x 4096 125, 104; but 512 against 28672 x 5120 (294 MB) 161, 178,
+// and 300 against 28672 x 4096 in tiles of 192 98, 144.
 constexpr float kSkPartial = 25.0f;
+constexpr long long kSkAllBytes = 150ll << 20;
 
 // How many of a launch's first tiles stream-K cuts into ranges: all when there are fewer than CTAs, else those of the incomplete last wave,
 // and a wave more where they are so few that many CTAs would share each of them.
@@ -28,22 +32,30 @@ inline int sk_cut_tiles(int tiles, int ctas) {
   return 2 * ctas > 7 * rest ? rest + ctas : rest;
 }
 
-// A launch's rule: the fix-up's cost, whether all tiles are cut, and whether stream-K may be chosen at all.
+// What the partials of the CTAs that share a tile cost, in k-blocks, when `cut` tiles are.
+inline float sk_partials(int cut, int sms) { return kSkPartial * (1.f + static_cast<float>(sms) / static_cast<float>(std::max(cut, 1))); }
+
+// A launch's rule: the fix-up's cost, whether all tiles are cut always, or where cutting the last does not pay, and whether stream-K may be
+// chosen at all.
 struct SkRule {
   float fix;
-  bool all, enabled;
-  int cut(int tiles, int sms) const { return all ? tiles : sk_cut_tiles(tiles, sms); }
+  bool all, all_else, enabled;
+  int cut(int tiles, int k_blocks, int sms) const {
+    const int last = all ? tiles : sk_cut_tiles(tiles, sms);
+    return all_else && !pays(tiles, last, k_blocks, sms) ? tiles : last;
+  }
+  // partials of the last tiles pass under the whole ones
+  static bool pays(int tiles, int cut, int k_blocks, int sms) { return cut == tiles || sk_partials(cut, sms) < 0.5f * static_cast<float>(k_blocks); }
 };
-inline SkRule sk_rule(bool scatter, bool tile_sums, bool enabled) { return SkRule{scatter ? kSkFixScatter : kSkFixPlain, scatter || tile_sums, enabled}; }
+inline SkRule sk_rule(bool scatter, bool tile_sums, bool enabled, int width, long long n, long long k) {
+  return SkRule{scatter ? kSkFixScatter : kSkFixPlain, scatter || tile_sums, width == 256 && n * k * 2 <= kSkAllBytes, enabled};
+}
 
 // The cost of the fix-ups of a launch, in k-blocks.
 inline float sk_fix(int tiles, int k_blocks, int sms, const SkRule& rule) {
-  const int cut = rule.cut(tiles, sms);
-  const float shared = static_cast<float>(sms) / static_cast<float>(std::max(cut, 1));
-  if (cut < tiles) {
-    const float own = kSkPartial * (1.f + shared);
-    return own < 0.5f * static_cast<float>(k_blocks) ? 0.25f * own : 1e6f;
-  }
+  const int cut = rule.cut(tiles, k_blocks, sms);
+  if (cut < tiles) return SkRule::pays(tiles, cut, k_blocks, sms) ? 0.25f * sk_partials(cut, sms) : 1e6f;
+  const float shared = static_cast<float>(sms) / static_cast<float>(tiles);
   return shared > kSkShared ? rule.fix * shared / kSkShared : rule.fix;
 }
 inline bool stream_k_applies(int tiles, int k_blocks, int sms, const SkRule& rule) {

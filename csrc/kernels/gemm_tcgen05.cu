@@ -740,13 +740,14 @@ static int launch_gemm(const void* A, const void* W, void* C, const void* bias, 
   uint32_t* sk_flags = nullptr;
   uint32_t sk_seq = 0;
   const int k_blocks = (K + kBK - 1) / kBK;
-  const SkRule rule = sk_rule(EPI == kEpiScatter, tile_sums(), stream_k_enabled());
+  const SkRule rule = sk_rule(EPI == kEpiScatter, tile_sums(), stream_k_enabled(), BN, N, K);
   batch.raster = group_tab == nullptr && batch.count == 1 && !rule.all && static_cast<long long>(M) * K * 2 > kRasterBytes;
   if (group_tab == nullptr && stream_k_applies(tiles, k_blocks, sms, rule)) {
     SkWorkspace* w = sk_workspace(stream, sms);
     if (w != nullptr) {
       grid = sms;
-      batch.cut = rule.cut(tiles, sms);
+      batch.cut = rule.cut(tiles, k_blocks, sms);
+      if (batch.cut == tiles && tiles > sms) batch.raster = 0;     // ranges over all tiles, in groups: 8192 rows against 2560 x 8192 281 -> 320 us
       sk_ws = w->ws;
       sk_flags = w->flags;
       sk_seq = ++w->seq;
@@ -933,7 +934,7 @@ static int gemm_bf16_dispatch(const void* A, const void* W, void* C, const void*
     for (int i = 0; i < 5; ++i) {
       if (cand[i] < 128 && m_tiles > 3) break;  // narrow tiles only pay off for decode-sized M
       const int tiles = m_tiles * ((N + cand[i] - 1) / cand[i]) * batch.count;
-      const float t = launch_cost(tiles, (K + kBK - 1) / kBK, sms, cost[i], sk_rule(false, tile_sums(), stream_k_enabled()));
+      const float t = launch_cost(tiles, (K + kBK - 1) / kBK, sms, cost[i], sk_rule(false, tile_sums(), stream_k_enabled(), cand[i], N, K));
       if (t < best - 1e-6f) { best = t; bn = cand[i]; }
     }
   }
@@ -1010,7 +1011,7 @@ extern "C" int ogb_gemm_bf16_scatter(const void* A, const void* W, int M, int N,
     bn = 256;
     for (int i = 0; i < 3; ++i) {
       const int tiles = m_tiles * ((N + cand[i] - 1) / cand[i]);
-      const float t = launch_cost(tiles, (K + kBK - 1) / kBK, sms, cost[i], sk_rule(true, tile_sums(), stream_k_enabled()));
+      const float t = launch_cost(tiles, (K + kBK - 1) / kBK, sms, cost[i], sk_rule(true, tile_sums(), stream_k_enabled(), cand[i], N, K));
       if (t < best - 1e-6f) { best = t; bn = cand[i]; }
     }
   }

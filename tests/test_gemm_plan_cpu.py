@@ -12,10 +12,11 @@ MAIN = r"""
 #include <cstdio>
 #include "gemm_plan.h"
 int main() {
-  int scatter, steady, enabled, tiles, kb, sms;
-  while (std::scanf("%d %d %d %d %d %d", &scatter, &steady, &enabled, &tiles, &kb, &sms) == 6) {
-    const ogb::SkRule r = ogb::sk_rule(scatter, steady, enabled);
-    std::printf("%d %d %.9g\n", ogb::stream_k_applies(tiles, kb, sms, r) ? 1 : 0, r.cut(tiles, sms), ogb::launch_cost(tiles, kb, sms, 1.f, r));
+  int scatter, steady, enabled, width, tiles, kb, sms;
+  long long n;
+  while (std::scanf("%d %d %d %d %lld %d %d %d", &scatter, &steady, &enabled, &width, &n, &tiles, &kb, &sms) == 8) {
+    const ogb::SkRule r = ogb::sk_rule(scatter, steady, enabled, width, n, kb * 64);
+    std::printf("%d %d %.9g\n", ogb::stream_k_applies(tiles, kb, sms, r) ? 1 : 0, r.cut(tiles, kb, sms), ogb::launch_cost(tiles, kb, sms, 1.f, r));
   }
 }
 """
@@ -52,21 +53,34 @@ SIZES = [(tiles, kb) for tiles in (1, 7, 24, 28, 100, 147, 148, 149, 160, 190, 1
 
 
 @pytest.mark.parametrize("scatter,steady,fix", [(1, 0, 13), (1, 1, 13), (0, 1, 40)])
-def test_all_tiles_are_cut(plan, scatter, steady, fix):
-    for (tiles, kb), (on, cut, cost) in zip(SIZES, plan([(scatter, steady, 1, t, kb, 148) for t, kb in SIZES])):
+@pytest.mark.parametrize("width,n", [(256, 1024), (256, 1 << 24), (128, 1024)])
+def test_all_tiles_are_cut(plan, scatter, steady, fix, width, n):
+    for (tiles, kb), (on, cut, cost) in zip(SIZES, plan([(scatter, steady, 1, width, n, t, kb, 148) for t, kb in SIZES])):
         want_on, want_cost = _ranges_over_all_tiles(fix, tiles, kb, 148)
         assert (on, cut) == (want_on, tiles), (tiles, kb)
         assert cost == pytest.approx(want_cost, rel=1e-6)
 
 
-def test_other_products_cut_the_last_wave(plan):
-    for (tiles, kb), (on, cut, cost) in zip(SIZES, plan([(0, 0, 1, t, kb, 148) for t, kb in SIZES])):
-        assert 0 < cut <= tiles or tiles % 148 == 0
-        assert (tiles - cut) % 148 == 0                         # whole waves follow
-        assert cut <= 148 + 148 * 2 // 7 + 1
+@pytest.mark.parametrize("width,n", [(256, 1024), (256, 1 << 24), (192, 1024)])
+def test_other_products_cut_the_last_wave(plan, width, n):
+    """Whole waves follow the cut tiles where their main loops are long enough to hide the fix-ups; elsewhere all tiles of full width over a weight
+    that stays in L2 are cut, and others are not."""
+    cuts = set()
+    for (tiles, kb), (on, cut, cost) in zip(SIZES, plan([(0, 0, 1, width, n, t, kb, 148) for t, kb in SIZES])):
+        rest = tiles % 148
+        last = tiles if tiles <= 148 else rest + 148 if 296 > 7 * rest else rest
+        hidden = last == tiles or 25 * (1 + 148 / max(last, 1)) < 0.5 * kb
+        all_else = width == 256 and n == 1024
+        assert cut == (tiles if not hidden and all_else else last), (tiles, kb)
         waves = -(-tiles // 148)
         assert cost <= waves and (on or cost == waves)
-    assert not any(on for on, _, _ in plan([(0, 0, 0, t, kb, 148) for t, kb in SIZES]))
+        if cut == tiles:
+            assert (on, cost) == pytest.approx(_ranges_over_all_tiles(40, tiles, kb, 148), rel=1e-6)
+        elif not hidden:
+            assert not on
+        cuts.add((on, cut < tiles))
+    assert cuts >= {(True, True), (True, False), (False, False)}
+    assert not any(on for on, _, _ in plan([(0, 0, 0, width, n, t, kb, 148) for t, kb in SIZES]))
 
 
 ROWS = r"""
