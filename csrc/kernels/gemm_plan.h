@@ -112,4 +112,27 @@ inline bool rows_applies(int m, int n, int k_blocks, bool gated, bool residual, 
   return m <= rows_limit((n + width - 1) / width, k_blocks, gated, residual, sms);
 }
 
+// int4 weights (gemm_w4a16.cu): `tiles` of 128 rows of W (of 128 gate and 128 up rows, when gated).  Against gemm_w4a16_tcgen05_kernel, which has
+// 64- or 128-column tiles, a CTA each, and its dequantisers' pace:
+//   gated: better at all sizes up to 160 rows but ranges of few k-blocks (896 x 40960 at 48 rows 38 -> 46)
+//   clusters of three CTAs and more per tile: 896 x 4864 37 -> 16 at 8 rows, 44 -> 21 at 256; 4096 x 896 14 -> 14 at 48, 15 -> 16 at 128
+//   two: 6144 x 4096 42 -> 31 at 8 rows, 33 -> 34 at 128, 41 -> 37 at 256; 6144 x 896 15 -> 14 at 8, 14 -> 16 at 64
+//   one: every CTA dequantises 128 rows where the other kernel's takes 64: 9728 x 4096 43 -> 49 at 8 rows, 43 -> 53 at 128; but that one has no 64-column
+//     tiles left to fill the SMs with beyond 14000, and up to 8 rows its 128-row tile costs: 14336 x 4096 51 -> 49, 18944 x 4096 66 -> 51
+//   ranges: up to 32 rows where the other kernel's last wave is short: 22016 x 4096 (172 tiles on 148 SMs) 76 -> 61 at 32 rows, at 48 76 -> 66;
+//     32000 x 2048 (250 tiles) 56 -> 49 at 16, 44 -> 49 at 32; up to 8 rows 32000 x 4096 111 -> 83; 896 in K 27 -> 29
+inline bool w4_rows_applies(int m, int tiles, int k_blocks, bool gated, int sms) {
+  if (m > kRowsMaxM) return false;
+  if (tiles > sms) {
+    if (m > kRowsRangesM) return false;
+    if (gated) return m <= kRowsGatedM || k_blocks >= 24;
+    if (k_blocks < 24) return false;
+    return m <= 8 || (4 * (tiles % sms) < sms && tiles < 2 * sms && (m <= 32 || k_blocks >= 48));
+  }
+  if (gated) return true;
+  if (tiles > sms / 2) return m <= 8 && 4 * tiles >= 3 * sms && k_blocks <= 96;
+  if (7 * tiles > 2 * sms) return k_blocks >= 48 || m <= 16;
+  return k_blocks >= 24 || m <= 64;
+}
+
 }  // namespace ogb

@@ -856,10 +856,14 @@ extern "C" int ogb_tile_sums(int on) {
   g_tile_sums = on != 0;
   return old;
 }
-// 1: a product of these sizes (gated: over N gate and up columns together) sums in ranges and takes a workspace.
-extern "C" int ogb_rows_in_ranges(int M, int N, int K, int gated) {
-  const int sms = ogb_num_sms(), width = gated != 0 ? 256 : 128;
-  return !tile_sums() && (N + width - 1) / width > sms && rows_applies(M, N, (K + kBK - 1) / kBK, gated != 0, false, sms) ? 1 : 0;
+// 1: a product of these sizes (kind 0: bf16, 1: bf16 gated over N gate and up columns together, 2 and 3: the same over int4 weights) sums in
+// ranges and takes a workspace.
+extern "C" int ogb_rows_in_ranges(int M, int N, int K, int kind) {
+  const bool gated = (kind & 1) != 0;
+  const int sms = ogb_num_sms(), tiles = gated ? (N / 2 + 127) / 128 : (N + 127) / 128, k_blocks = (K + kBK - 1) / kBK;
+  if (tiles <= sms) return 0;
+  if (kind >= 2) return w4_rows_applies(M, tiles, k_blocks, gated, sms) ? 1 : 0;
+  return !tile_sums() && rows_applies(M, N, k_blocks, gated, false, sms) ? 1 : 0;
 }
 extern "C" int64_t ogb_rows_counter_bytes(void) { return static_cast<int64_t>(rows_counter_bytes(ogb_num_sms())); }
 extern "C" int64_t ogb_rows_workspace_bytes(int rows) {

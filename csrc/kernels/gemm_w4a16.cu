@@ -372,7 +372,7 @@ gemm_w4a16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const uint
 }
 
 // ------------------------------------------------------------------------------------------
-// Few rows (M <= kRowsMaxM): the scheme of gemm_rows.cuh over int4 weights.  A decode step of a small model is bound by the chain
+// Few rows (w4_rows_applies in gemm_plan.h): the scheme of gemm_rows.cuh over int4 weights.  A decode step of a small model is bound by the chain
 // load -> dequantise -> multiply of a few CTAs, not by bytes: 64 rows against a 896 x 4864 projection left 14 CTAs to walk 76 k-blocks one
 // after the other (33 us for 2.3 MB).  Here 128 dequantised rows of W are the M side of the MMA, the activations its N side, and a
 // cluster shares the k-blocks of a tile (2 - 10 each at these sizes, whose loads are under way before the first is used).  The gated
@@ -526,7 +526,6 @@ static int launch_w4_rows_one(const void* x, int K, int ldx, RowsGemmParams p, W
   p.n_tiles = (wp.tile_rows + kWTile - 1) / kWTile;
   int grid, smem;
   if (p.n_tiles > sms) {
-    if (p.M > kRowsRangesM) return kRowsDeclined;
     p.splits = 0;
     grid = sms;
     p.stages = std::min(kRowsMaxStages, (kRowsSmemMax - kRowsBarBytes - TW * kRowsStage) / stage_bytes);
@@ -597,7 +596,7 @@ extern "C" int ogb_w4a16_gemm(const void* x, const void* qweight, const void* sc
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((K % 32) != 0 || (ldx % 8) != 0 || (ldc % 8) != 0) return -3;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(qweight)) & 15) return -4;
-  if (M <= kRowsMaxM) {
+  if (w4_rows_applies(M, (N + kWTile - 1) / kWTile, (K + kWBK - 1) / kWBK, false, ogb_num_sms())) {
     const int rc = launch_w4_rows(x, qweight, scales, zp, bias, out, M, N, K, ldx, ldc, scales_f32 != 0, false, status, stream);
     if (rc != kRowsDeclined) return rc;
   }
@@ -618,12 +617,13 @@ extern "C" int ogb_w4a16_gemm(const void* x, const void* qweight, const void* sc
 }
 
 // out[M, N / 2] = silu(gate) * up of a projection whose first N / 2 rows are the gate's and the others the up projection's; arguments as
-// above, without a bias.  M at most 256.  -11: not here (more tiles than SMs, and no workspace or many rows).
+// above, without a bias.  M at most 256.  -11: not here (more tiles than SMs, and no workspace, many rows or a short K).
 extern "C" int ogb_w4a16_gated(const void* x, const void* qweight, const void* scales, const void* zp, void* out, int M, int N, int K, int ldx, int ldc,
                                int scales_f32, int* status, void* stream_) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (M > kRowsMaxM || (N % 2) != 0 || (K % 32) != 0 || (ldx % 8) != 0 || (ldc % 8) != 0) return -3;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(qweight)) & 15) return -4;
+  if (!w4_rows_applies(M, (N / 2 + kWTile - 1) / kWTile, (K + kWBK - 1) / kWBK, true, ogb_num_sms())) return -11;
   const int rc = launch_w4_rows(x, qweight, scales, zp, nullptr, out, M, N, K, ldx, ldc, scales_f32 != 0, true, status, static_cast<cudaStream_t>(stream_));
   return rc == kRowsDeclined ? -11 : rc;
 }

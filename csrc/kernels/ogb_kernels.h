@@ -25,8 +25,9 @@ int ogb_gemm_bf16(const void* A, const void* W, void* C, const void* bias, const
 void ogb_launch_scope(void* ws, int64_t bytes, int overlap);
 int64_t ogb_rows_workspace_bytes(int rows);
 int64_t ogb_rows_counter_bytes(void);
-// 1: a product of these sizes (gated: N gate and up columns together) takes a workspace.
-int ogb_rows_in_ranges(int M, int N, int K, int gated);
+// 1: a product of these sizes (kind 0: bf16, 1: bf16 gated over N gate and up columns together, 2 and 3: the same over int4 weights) takes a
+// workspace.
+int ogb_rows_in_ranges(int M, int N, int K, int kind);
 // on != 0: products that the calling thread launches from now on sum over K as the tile kernel alone does, whatever their rows (models
 // that choose among experts).  Returns the old setting.
 int ogb_tile_sums(int on);

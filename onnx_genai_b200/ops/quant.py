@@ -5,7 +5,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _native, call_scope, in_order, launch_counts, num_sms, reference, status_word, timed_region
+from . import _native, call_scope, in_order, launch_counts, reference, status_word, timed_region
 from . import gemm as _gemm
 
 GEMV_MAX_M = 8          # rows the GEMV kernels accept
@@ -89,8 +89,9 @@ class QuantLinear:
         if (not x.is_cuda or not FUSED_MAX_M < m <= GATED_MAX_M or self.bias is not None or self.large_m != "int4" or self.n % 2 or self.k % 32
                 or x.stride(1) != 1 or x.stride(0) % 8 or out.stride(0) % 8 or _LEGACY_GEMV):
             return False
-        with timed_region("w4a16_gemm"), call_scope(m, lambda: self.n > 256 * num_sms(), x.device):
-            rc = _native.load().ogb_w4a16_gated(x.data_ptr(), self.qweight.data_ptr(), self.scales.data_ptr(), self.zp.data_ptr() if self.zp is not None else 0,
+        lib = _native.load()
+        with timed_region("w4a16_gemm"), call_scope(m, lambda: lib.ogb_rows_in_ranges(m, self.n, self.k, 3), x.device):
+            rc = lib.ogb_w4a16_gated(x.data_ptr(), self.qweight.data_ptr(), self.scales.data_ptr(), self.zp.data_ptr() if self.zp is not None else 0,
                                                 out.data_ptr(), m, self.n, self.k, x.stride(0), out.stride(0), int(self.scales_fp32),
                                                 status_word(x.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
         if rc == _NO_WORKSPACE:
@@ -131,7 +132,7 @@ class QuantLinear:
             launch_counts["w4a16_gemv"] += 1
             return out
         if self.large_m == "int4" and self.k % 32 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and out.stride(0) % 8 == 0:
-            with timed_region("w4a16_gemm"), call_scope(m, lambda: self.n > 128 * num_sms(), x.device):
+            with timed_region("w4a16_gemm"), call_scope(m, lambda: lib.ogb_rows_in_ranges(m, self.n, self.k, 2), x.device):
                 rc = lib.ogb_w4a16_gemm(x.data_ptr(), self.qweight.data_ptr(), self.scales.data_ptr(),
                                         self.zp.data_ptr() if self.zp is not None else 0,
                                         self.bias.data_ptr() if self.bias is not None else 0, out.data_ptr(), m, self.n, self.k,

@@ -130,3 +130,32 @@ def test_few_rows_have_their_own_kernel_where_that_is_faster(rows, size):
 
 def test_sums_with_a_residual_stay_where_they_are_rounded_once(rows):
     assert all(rows(256, n, k, False, True) for n, k in [(128, 64), (3584, 512), (896, 896), (4608, 18944)])
+
+
+W4 = r"""
+#include <cstdio>
+#include "gemm_plan.h"
+int main() {
+  int m, tiles, kb, gated, sms;
+  while (std::scanf("%d %d %d %d %d", &m, &tiles, &kb, &gated, &sms) == 5) std::printf("%d\n", ogb::w4_rows_applies(m, tiles, kb, gated, sms) ? 1 : 0);
+}
+"""
+
+
+# (rows, rows of W, K, gated, the kernels for few rows): 1.1 to 1.34 times the other kernel's time, or 0.33 to 0.9 of it
+@pytest.mark.parametrize("m,n,k,gated,few", [
+    (48, 32000, 896, 0, 0), (128, 14336, 2048, 0, 0), (128, 9728, 896, 0, 0), (128, 18944, 4096, 0, 0), (16, 9728, 4096, 0, 0), (8, 11008, 11008, 0, 0),
+    (64, 6144, 896, 0, 0), (64, 6144, 2048, 0, 0), (48, 22016, 896, 0, 0), (48, 22016, 2048, 0, 0), (48, 40960, 896, 1, 0), (300, 896, 4864, 0, 0),
+    (8, 896, 4864, 0, 1), (256, 4096, 4096, 0, 1), (48, 896, 896, 0, 1), (64, 1152, 896, 0, 1), (256, 6144, 11008, 0, 1), (8, 18944, 4096, 0, 1),
+    (32, 22016, 4096, 0, 1), (48, 22016, 4864, 0, 1), (8, 32000, 4096, 0, 1), (64, 9728, 896, 1, 1), (160, 9728, 896, 1, 1), (16, 40960, 896, 1, 1)])
+def test_int4_products_of_few_rows(tmp_path_factory, m, n, k, gated, few):
+    if shutil.which("g++") is None:
+        pytest.skip("needs g++")
+    d = tmp_path_factory.getbasetemp() / "w4"
+    if not (d / "main").exists():
+        d.mkdir()
+        (d / "main.cpp").write_text(W4)
+        subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(KERNELS), str(d / "main.cpp"), "-o", str(d / "main")], check=True)
+    tiles = -(-n // (2 if gated else 1) // 128)
+    out = subprocess.run([str(d / "main")], input=f"{m} {tiles} {-(-k // 64)} {gated} 148", capture_output=True, text=True, check=True).stdout
+    assert out.strip() == str(few)
