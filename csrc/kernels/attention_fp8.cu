@@ -15,11 +15,13 @@
 #include <cooperative_groups.h>
 #include <cuda_fp8.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <mutex>
 #include <unordered_map>
 
 #include "attention_common.cuh"
+#include "attention_plan.h"
 #include "ogb_kernels.h"
 
 namespace ogb {
@@ -742,9 +744,9 @@ __global__ void __maxnreg__(168) paged_decode_e4m3_mma_kernel(const __grid_const
 // prefill (chunked, causal): 64 query rows x one head per CTA; the four consumer warps expand each
 // 64-key block together into one shared bf16 tile.
 // A tile with at most 32 rows takes 2, 4 or 8 heads of its KV head (64 accumulator rows = heads x 32, 16 or 8 query rows), so a
-// short turn against a long context expands the context once for several heads.  Where that leaves few CTAs, a cluster of
-// num_splits CTAs shares a tile: each walks a part of the keys, then each merges a part of the rows out of all their shared memories
-// (16 rows against 6000 - 12000 tokens, 8 sequences, 28 heads over 4: 1125 -> 290 us; int8, 16 sequences of 300 - 2300: 229 -> 74).
+// short turn against a long context expands the context once for several heads.  Where that leaves few CTAs (attention_plan.h), those of a
+// cluster share a tile: each walks a part of the keys, then each merges a part of the rows out of all their shared memories
+// (16 rows against 6000 - 12000 tokens, 8 sequences, 28 heads over 4: 1087 -> 327 us; 16 sequences of 300 - 2300: 299 -> 130).
 // ------------------------------------------------------------------------------------------
 constexpr int kPreStages = 2;
 constexpr int kPreTile = kKvBlock * kD * 2;   // 16 KB bf16 K tile (and as much for V)
@@ -763,8 +765,8 @@ __global__ void __launch_bounds__(kAttnThreads) paged_prefill_fp8_kernel(const _
   float* sc_sh = reinterpret_cast<float*>(empty_bar + kPreStages);   // [4 pages][2]
 
   namespace cg = cooperative_groups;
-  const int splits = p.num_splits, split = blockIdx.x % splits;      // the cluster's size and this CTA's place in it
-  const int tile = blockIdx.x / splits;
+  const int split = blockIdx.x % p.num_splits;                       // this CTA's place in its cluster
+  const int tile = blockIdx.x / p.num_splits;
   if (tile >= p.num_tiles) return;
   const int head = blockIdx.y, kvh = head / p.group;
   const int seq = p.tile_seq[tile], q0 = p.tile_q0[tile];
@@ -774,12 +776,14 @@ __global__ void __launch_bounds__(kAttnThreads) paged_prefill_fp8_kernel(const _
   const int rows = min(64, q_len - q0);
   const int pos0 = ctx - q_len + q0;
   if (rows <= 0 || ctx <= 0) return;
-  const int row_bits = rows > 32 ? 6 : rows > 16 ? 5 : rows > 8 ? 4 : 3;
+  const int row_bits = prefill_row_bits(rows);
   if ((head % p.group) & ((64 >> row_bits) - 1)) return;               // served with an earlier head of the group
   const int heads_here = min(64 >> row_bits, p.group - head % p.group);
   const int kv_end = min(ctx, pos0 + rows);
   const int kv_lo = (p.window > 0) ? max(0, pos0 - p.window + 1) : 0;   // first key any row of the tile sees in its window
   const int blocks = (kv_end + kKvBlock - 1) / kKvBlock;
+  const int splits = prefill_shares(p.num_splits, blocks);           // the CTAs that share this tile; cluster barriers count no others
+  if (split >= splits) return;
   const int b_begin = blocks * split / splits, b_end = blocks * (split + 1) / splits;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -1066,7 +1070,7 @@ static int launch_decode_q(const void* q, void* out, const void* pool, const flo
 
 static int launch_prefill_q(const void* q, void* out, const void* pool, const float* scales, int kv_fmt, const int* page_table,
                             const int* ctx_len, const int* cu_q, const int* tile_seq, const int* tile_q0, int num_tiles,
-                            int num_seqs, int max_pages, int64_t num_pages, int hq, int hkv, int d, int q_stride,
+                            int num_seqs, int q_rows, int max_keys, int max_pages, int64_t num_pages, int hq, int hkv, int d, int q_stride,
                             int o_stride, float scale, int window, int sink, int* status, void* stream) {
   if (num_tiles <= 0) return 0;
   if (kv_fmt < 0 || kv_fmt > 2) return -3;
@@ -1084,11 +1088,10 @@ static int launch_prefill_q(const void* q, void* out, const void* pool, const fl
     OGB_CUDA_CHECK(cudaFuncSetAttribute(paged_prefill_fp8_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     attr_set = true;
   }
-  // A tile's CTAs if it has at most 16 rows (longer tiles bring more and have the keys' work to themselves all the same): share
-  // the keys among as many CTAs as two per SM leave room for.  8-byte stores of the merge want an even output stride.
-  const int ctas = num_tiles * hkv * ((p.group + 3) / 4);
-  int splits = 1;
-  while (!tile_sums() && splits < 8 && 2 * splits * ctas <= 2 * ogb_num_sms() && (o_stride % 4) == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0) splits *= 2;
+  // 8-byte stores of the merge want an even output stride
+  const bool shares = !tile_sums() && (o_stride % 4) == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
+  const int splits = shares ? prefill_splits(num_tiles, q_rows, hkv, p.group, std::min<long long>(max_keys, static_cast<long long>(max_pages) * kPageTokens), ogb_num_sms())
+                            : 1;
   p.num_splits = splits;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(num_tiles * splits, hq);
@@ -1115,7 +1118,7 @@ extern "C" int ogb_paged_prefill_fp8(const void* q, void* out, const void* pool,
                                      const int* ctx_len, const int* cu_q, const int* tile_seq, const int* tile_q0, int num_tiles,
                                      int num_seqs, int max_pages, int64_t num_pages, int hq, int hkv, int d, int q_stride,
                                      int o_stride, float scale, int* status, void* stream) {
-  return launch_prefill_q(q, out, pool, scales, 0, page_table, ctx_len, cu_q, tile_seq, tile_q0, num_tiles, num_seqs, max_pages,
+  return launch_prefill_q(q, out, pool, scales, 0, page_table, ctx_len, cu_q, tile_seq, tile_q0, num_tiles, num_seqs, 64 * num_tiles, INT32_MAX, max_pages,
                           num_pages, hq, hkv, d, q_stride, o_stride, scale, 0, 0, status, stream);
 }
 // One-byte pages in any format: kv_format 0 = e4m3, 1 = int8 (symmetric), 2 = e5m2; same per-(page, head, K|V) scale layout.
@@ -1128,9 +1131,9 @@ extern "C" int ogb_paged_decode_q8(const void* q, void* out, const void* pool, c
 }
 extern "C" int ogb_paged_prefill_q8(const void* q, void* out, const void* pool, const float* scales, int kv_format,
                                     const int* page_table, const int* ctx_len, const int* cu_q, const int* tile_seq,
-                                    const int* tile_q0, int num_tiles, int num_seqs, int max_pages, int64_t num_pages, int hq,
+                                    const int* tile_q0, int num_tiles, int num_seqs, int q_rows, int max_keys, int max_pages, int64_t num_pages, int hq,
                                     int hkv, int d, int q_stride, int o_stride, float scale, int window, int sink, int* status,
                                     void* stream) {
-  return launch_prefill_q(q, out, pool, scales, kv_format, page_table, ctx_len, cu_q, tile_seq, tile_q0, num_tiles, num_seqs,
+  return launch_prefill_q(q, out, pool, scales, kv_format, page_table, ctx_len, cu_q, tile_seq, tile_q0, num_tiles, num_seqs, q_rows, max_keys,
                           max_pages, num_pages, hq, hkv, d, q_stride, o_stride, scale, window, sink, status, stream);
 }

@@ -110,7 +110,8 @@ int ogb_paged_prefill_fp8(const void* q, void* out, const void* pool, const floa
                           int num_seqs, int max_pages, int64_t num_pages, int hq, int hkv, int d, int q_stride, int o_stride,
                           float scale, int* status, void* stream);
 
-// One-byte pages (kv_format 0 = e4m3, 1 = symmetric int8, 2 = e5m2), same pool and scale layout.
+// One-byte pages (kv_format 0 = e4m3, 1 = symmetric int8, 2 = e5m2), same pool and scale layout.  q_rows: query rows of all tiles together;
+// max_keys: what no context is longer than, as far as the caller knows.
 int ogb_rope_kv_append_q8(void* qkv, const int* positions, const int* slots, const float* cos_sin, void* pool, float* scales,
                           int kv_format, int tokens, int hq, int hkv, int d, int rotary_dim, int interleaved, int page_size,
                           int64_t num_slots, int max_pos, int* status, void* stream);
@@ -124,7 +125,7 @@ int ogb_paged_decode_q8(const void* q, void* out, const void* pool, const float*
                         int sink, int* status, void* stream);
 int ogb_paged_prefill_q8(const void* q, void* out, const void* pool, const float* scales, int kv_format, const int* page_table,
                          const int* ctx_len, const int* cu_q, const int* tile_seq, const int* tile_q0, int num_tiles,
-                         int num_seqs, int max_pages, int64_t num_pages, int hq, int hkv, int d, int q_stride, int o_stride,
+                         int num_seqs, int q_rows, int max_keys, int max_pages, int64_t num_pages, int hq, int hkv, int d, int q_stride, int o_stride,
                          float scale, int window, int sink, int* status, void* stream);
 
 // Sampling.  logits [rows, vocab] bf16 (ld = row stride).  out_tokens int32 [rows].

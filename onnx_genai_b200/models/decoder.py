@@ -567,7 +567,7 @@ class DecoderModel:
                     np_ = si.num_prefill_seqs
                     ops.paged_prefill(qkv[nd:], attn[nd:], pool, si.page_table[nd:nd + np_], si.ctx_len[nd:nd + np_],
                                       si.cu_q, si.tile_seq, si.tile_q0, si.num_tiles, self.hq, self.hkv, self.d, self.scale,
-                                      cfg.sliding_window, kv_scales=kv.scales[li] if kv.scales is not None else None, sink=cfg.sink_len)
+                                      cfg.sliding_window, kv_scales=kv.scales[li] if kv.scales is not None else None, sink=cfg.sink_len, max_ctx=si.max_ctx)
                 lw.quant["o"].fused(attn, x, residual=x)
                 gu = self.gate_up[:t, : 2 * lw.quant["gate"].n]
                 lw.quant["gate_up"].fused(x, gu, norm_weight=lw.ln2, eps=cfg.rms_eps)
@@ -599,7 +599,7 @@ class DecoderModel:
                 np_ = si.num_prefill_seqs
                 ops.paged_prefill(qkv[nd:], attn[nd:], pool, si.page_table[nd:nd + np_], si.ctx_len[nd:nd + np_],
                                   si.cu_q, si.tile_seq, si.tile_q0, si.num_tiles, self.hq, self.hkv, self.d, self.scale,
-                                  cfg.sliding_window, kv_scales=kv.scales[li] if kv.scales is not None else None, sink=cfg.sink_len)
+                                  cfg.sliding_window, kv_scales=kv.scales[li] if kv.scales is not None else None, sink=cfg.sink_len, max_ctx=si.max_ctx)
             if lw.quant:
                 pending = lw.quant["o"](attn, out=self.partial[:t])
                 self._norm(x, lw.ln2, pending, h)
@@ -661,7 +661,7 @@ class DecoderModel:
             np_ = si.num_prefill_seqs
             ops.paged_prefill(qkv[nd:], attn[nd:], pool, si.page_table[nd:nd + np_], si.ctx_len[nd:nd + np_],
                               si.cu_q, si.tile_seq, si.tile_q0, si.num_tiles, self.hq, self.hkv, self.d, self.scale,
-                              cfg.sliding_window, kv_scales=scales, sink=cfg.sink_len)
+                              cfg.sliding_window, kv_scales=scales, sink=cfg.sink_len, max_ctx=si.max_ctx)
 
     def _forward_tp_fused(self, si: StepInputs, kv: "KVCache") -> torch.Tensor:
         """The step under fused tensor parallelism, driven op by op (the C++ executor runs the same sequence).

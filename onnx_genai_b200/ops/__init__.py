@@ -423,9 +423,10 @@ def prefill_tiles(q_lens, block_m=64):
 
 @_timed("paged_prefill")
 def paged_prefill(q, out, pool, page_table, ctx_len, cu_q, tile_seq, tile_q0, num_tiles, hq, hkv, d, scale=None,
-                  window=0, kv_scales=None, sink=0):
+                  window=0, kv_scales=None, sink=0, max_ctx=None):
     """Causal varlen GQA over paged KV for chunks of new tokens.  q: packed qkv rows (first hq*d cols).
-    ``kv_scales`` selects the e4m3 page kernels."""
+    ``kv_scales`` selects the e4m3 page kernels.  ``max_ctx``: what no context is longer than, where the caller knows (how the work is
+    divided depends on it, not the result)."""
     scale = scale or 1.0 / math.sqrt(d)
     if not q.is_cuda:
         if kv_scales is None and _cpu_native(q) and pool.dtype == torch.float32 and pool.is_contiguous():
@@ -436,8 +437,8 @@ def paged_prefill(q, out, pool, page_table, ctx_len, cu_q, tile_seq, tile_q0, nu
     if kv_scales is not None:
         rc = _native.load().ogb_paged_prefill_q8(
             q.data_ptr(), out.data_ptr(), pool.data_ptr(), kv_scales.data_ptr(), kv_format(pool), page_table.data_ptr(), ctx_len.data_ptr(),
-            cu_q.data_ptr(), tile_seq.data_ptr(), tile_q0.data_ptr(), int(num_tiles), ctx_len.numel(), page_table.shape[1],
-            backed_pages(pool), hq, hkv, d, q.stride(0), out.stride(0), float(scale), int(window), int(sink), status_word().data_ptr(),
+            cu_q.data_ptr(), tile_seq.data_ptr(), tile_q0.data_ptr(), int(num_tiles), ctx_len.numel(), q.shape[0],
+            int(max_ctx) if max_ctx else 0x7fffffff, page_table.shape[1], backed_pages(pool), hq, hkv, d, q.stride(0), out.stride(0), float(scale), int(window), int(sink), status_word().data_ptr(),
             _stream())
         _native.check(rc, "ogb_paged_prefill_q8")
         launch_counts["paged_prefill_fp8"] += 1

@@ -44,7 +44,7 @@ _SIGNATURES = {
     "ogb_paged_prefill_fp8": ([P, P, P, P, P, P, P, P, P, I, I, I, L, I, I, I, I, I, F, P, P], I),
     "ogb_rope_kv_append_q8": ([P, P, P, P, P, P, I, I, I, I, I, I, I, I, L, I, P, P], I),
     "ogb_paged_decode_q8": ([P, P, P, P, I, P, P, I, I, L, I, I, I, I, I, F, I, P, P, I, I, P, P], I),
-    "ogb_paged_prefill_q8": ([P, P, P, P, I, P, P, P, P, P, I, I, I, L, I, I, I, I, I, F, I, I, P, P], I),
+    "ogb_paged_prefill_q8": ([P, P, P, P, I, P, P, P, P, P, I, I, I, I, I, L, I, I, I, I, I, F, I, I, P, P], I),
     "ogb_gemm_bf16_batched": ([P, P, P, I, I, I, I, I, I, I, I, I, P, P], I),
     "ogb_gemm_f32": ([P, P, P, I, I, I, I, I, I, I, I, I, P], I),
     "ogb_argmax_f32": ([P, P, I, I, I, P], I),
