@@ -78,6 +78,7 @@ struct AttnParams {
   int window;               // > 0: a query sees only the last `window` keys ...
   int sink;                 // ... and, with window > 0, the first `sink` keys as well (attention sinks)
   int num_splits;
+  int pack_heads;           // prompts on the tensor cores: a tile with few rows takes several heads of its KV head
   int cluster_merge;        // decode: the splits of a row are a cluster that merges them itself (no part_o, no part_ml)
   float* part_o;
   float* part_ml;

@@ -180,8 +180,10 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
   if (rows <= 0 || ctx <= 0) return;
   // A tile with few rows takes several query heads of its KV head: 1 << row_bits tile rows per head.  The later turn of a
   // conversation -- at most 16 new tokens against a long context -- then reads the context once for 8 heads instead of 8 times
-  // with 16 of 128 rows in use (256 sequences of 614 tokens and 16 rows each, 28 heads over 4: 895 -> 177 us).
-  const int row_bits = CHUNKED || rows > 64 ? 7 : rows > 32 ? 6 : rows > 16 ? 5 : 4;
+  // with 16 of 128 rows in use (256 sequences of 614 tokens and 16 rows each, 28 heads over 4: 895 -> 177 us).  p.pack_heads: not where each
+  // head's CTAs have an SM of their own anyway, nor where a KV head has one query head (the rows come in smaller pieces: 25 -> 29 us for 64 rows of
+  // 1000 tokens, 16 heads over 16: 238 -> 254 for 256 sequences of 100).
+  const int row_bits = CHUNKED || p.pack_heads == 0 || rows > 64 ? 7 : rows > 32 ? 6 : rows > 16 ? 5 : 4;
   const int heads_here = min(kFaBM >> row_bits, p.group - head % p.group);
   if ((head % p.group) & ((kFaBM >> row_bits) - 1)) return;        // served with an earlier head of the group
   const int kv_end = min(ctx, pos0 + rows);
@@ -598,8 +600,10 @@ static int launch_prefill_tc(const AttnParams& p, const void* pool, int q_rows, 
     attr_set = true;
   }
   dim3 grid(p.num_tiles, p.hq);
+  AttnParams pl = p;
+  pl.pack_heads = p.group > 1 && static_cast<long long>(grid.x) * grid.y > ogb_num_sms();
   return static_cast<int>(launch_overlapped(paged_prefill_tc_kernel<DK, DV, BN, CHUNKED>, grid, dim3(kFaThreads), Cfg::kSmemBytes, stream, q_map, q16_map,
-                                            kv_map, p));
+                                            kv_map, pl));
 }
 
 static unsigned long long* g_fa_dbg = nullptr;
