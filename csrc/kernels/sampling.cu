@@ -12,6 +12,7 @@
 // argmax ties go to the lowest token id (crates/onnx-genai-engine/src/sampling.rs:120-132).
 #include "common.cuh"
 #include "ogb_kernels.h"
+#include "sampling_plan.h"
 
 namespace ogb {
 
@@ -276,8 +277,8 @@ sample_kernel(const T* __restrict__ logits, int* __restrict__ out, const float* 
 // ------------------------------------------------------------------------------------------
 // Vectorised variant of sample_kernel: identical arithmetic and results, but every pass over the
 // row uses 16-byte loads (8 logits or 4 weights per thread per iteration), so a pass costs ~4x fewer
-// dependent memory round trips.  Requires vocab % 8 == 0, ld % 8 == 0 and 16-byte aligned rows.  For vocabularies beyond what a
-// cluster holds (sample_cluster_kernel).
+// dependent memory round trips.  Requires vocab % 8 == 0, ld % 8 == 0 and 16-byte aligned rows.  For many rows of a short
+// vocabulary (sampling_plan.h), and vocabularies beyond what a cluster holds.
 // ------------------------------------------------------------------------------------------
 template <bool BY_MASS>
 OGB_DEVICE uint32_t radix_threshold_vec(const uint32_t* __restrict__ w, int vocab, uint32_t floor_w,
@@ -597,23 +598,29 @@ extern "C" int ogb_argmax_bf16(const void* logits, int* out_tokens, int rows, in
   return static_cast<int>(cudaGetLastError());
 }
 
+// All three kernels pick the same tokens.
+static int sample_rows(const void* logits, int* out_tokens, const float* temperature, const int* top_k, const float* top_p, const float* min_p,
+                       const float* uniform, uint32_t* work, int rows, int vocab, int ld, cudaStream_t stream) {
+  const bool vec_ok = (vocab % 8 == 0) && (ld % 8 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0) &&
+                      ((reinterpret_cast<uintptr_t>(work) & 15) == 0);
+  if (sample_cluster_applies(logits, vocab, ld) && (sample_cluster_pays(rows, vocab) || !vec_ok))
+    return launch_sample_cluster(logits, out_tokens, temperature, top_k, top_p, min_p, uniform, rows, vocab, ld, stream);
+  if (vec_ok) {
+    sample_kernel_vec<<<rows, kSampleThreads, 0, stream>>>(static_cast<const __nv_bfloat16*>(logits), out_tokens, temperature, top_k, top_p, min_p, uniform,
+                                                           work, vocab, ld);
+  } else {
+    sample_kernel<<<rows, kSampleThreads, 0, stream>>>(static_cast<const __nv_bfloat16*>(logits), out_tokens, temperature, top_k, top_p, min_p, uniform, work,
+                                                       vocab, ld);
+  }
+  return static_cast<int>(cudaGetLastError());
+}
+
 extern "C" int ogb_sample_bf16(const void* logits, int* out_tokens, const float* temperature, const int* top_k,
                                const float* top_p, const float* min_p, const float* uniform, uint32_t* work, int rows,
                                int vocab, int ld, void* stream) {
   if (rows <= 0) return 0;
   if (work == nullptr) return -4;
-  if (sample_cluster_applies(logits, vocab, ld))
-    return launch_sample_cluster(logits, out_tokens, temperature, top_k, top_p, min_p, uniform, rows, vocab, ld, static_cast<cudaStream_t>(stream));
-  const bool vec_ok = (vocab % 8 == 0) && (ld % 8 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0) &&
-                      ((reinterpret_cast<uintptr_t>(work) & 15) == 0);
-  if (vec_ok) {
-    sample_kernel_vec<<<rows, kSampleThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(logits), out_tokens, temperature, top_k, top_p, min_p, uniform, work, vocab, ld);
-    return static_cast<int>(cudaGetLastError());
-  }
-  sample_kernel<<<rows, kSampleThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(logits), out_tokens, temperature, top_k, top_p, min_p, uniform, work, vocab, ld);
-  return static_cast<int>(cudaGetLastError());
+  return sample_rows(logits, out_tokens, temperature, top_k, top_p, min_p, uniform, work, rows, vocab, ld, static_cast<cudaStream_t>(stream));
 }
 
 // The same over fp32 logits (the 32-bit engine).
@@ -670,13 +677,6 @@ extern "C" int ogb_sample_bf16_no_alloc(const void* logits, int* out_tokens, con
     if (e != cudaSuccess) return static_cast<int>(e);
     g_no_alloc_work_ptr[dev] = static_cast<uint32_t*>(p);
   }
-  // same choice as ogb_sample_bf16 (kNoAllocMaxVocab logits always fit the cluster); both kernels pick identical tokens
-  if (sample_cluster_applies(logits, vocab, ld)) {
-    return launch_sample_cluster(logits, out_tokens, temperature, top_k, top_p, min_p, uniform, rows, vocab, ld, static_cast<cudaStream_t>(stream));
-  } else {
-    sample_kernel<<<rows, kSampleThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(logits), out_tokens, temperature, top_k, top_p, min_p, uniform,
-        g_no_alloc_work_ptr[dev], vocab, ld);
-  }
-  return static_cast<int>(cudaGetLastError());
+  return sample_rows(logits, out_tokens, temperature, top_k, top_p, min_p, uniform, g_no_alloc_work_ptr[dev], rows, vocab, ld,
+                     static_cast<cudaStream_t>(stream));
 }
