@@ -17,6 +17,9 @@ _native.register("ogb_grouped_gemm_act", [P] * 5 + [I] * 9 + [F, F, I, P, P])
 _native.register("ogb_grouped_gemm_f32", [P] * 5 + [I] * 8 + [F, F, P])
 
 
+PERMUTE_ONE_ROUTES = 4096        # routes up to which the permutation is one launch (moe.cu), for the launch counts
+
+
 def _stream():
     return torch.cuda.current_stream().cuda_stream
 
@@ -100,7 +103,7 @@ def moe_experts(h, router_logits, expert_gate_up, expert_down, ws: MoEWorkspace,
                                  int(accumulate), s)
     _native.check(rc, "ogb_moe_combine")
     launch_counts["moe_route_topk"] += 1
-    launch_counts["moe_permute"] += 4
+    launch_counts["moe_permute"] += 1 if t * k <= PERMUTE_ONE_ROUTES else 4
     launch_counts["moe_gather_rows"] += 1
     launch_counts["moe_grouped_gemm"] += 2
     launch_counts["moe_combine"] += 1
@@ -164,7 +167,7 @@ def routed_experts(h, logits, up, down, ws: MoEWorkspace, k, act, half=0, groups
                                               w.shape[2], c.stride(0), *f.args, 2 * half if f.gated else 0, st, s)
         _native.check(rc, "grouped product " + name)
     launch_counts["moe_route_topk"] += 1
-    launch_counts["moe_permute"] += 4
+    launch_counts["moe_permute"] += 1 if t * k <= PERMUTE_ONE_ROUTES else 4
     launch_counts["moe_gather_rows"] += 1
     launch_counts["moe_grouped_gemm"] += 2
     return ExpertRows(ys, ws.route_pos[: t * k].view(t, k), ws.topk_w[: t * k].view(t, k))
